@@ -68,7 +68,7 @@ def draw(rng):
     what = rng.choice(("decode", "batch", "prompt", "gemv", "gemm", "prefill", "prefill", "q8", "q8_signed"))
     group = rng.choice((32, 64, 64, 64, 128))
     if what in ("decode", "batch", "prompt"):
-        m = {"decode": 1, "batch": rng.randint(2, 8), "prompt": _between(rng, 9, 480)}[what]
+        m = {"decode": 1, "batch": rng.randint(2, 8), "prompt": _between(rng, 9, 420)}[what]
         hidden = rng.choice((1024, 2048, 4096)) if m == 1 else _between(rng, 1024, 5120, 256)
         inter = _between(rng, max(2 * hidden, 4352), max(4 * hidden, 6144) if hidden <= 4096 else 17408, 256)
         c = _layers("", m, hidden, inter, _between(rng, 1024, 4096, 256),
