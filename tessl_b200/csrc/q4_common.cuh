@@ -28,6 +28,23 @@ __device__ __forceinline__ uint32_t ldg_stream4(const void *p)
     return v;
 }
 
+/// Loads of data that the preceding kernel of the stream may have written, for kernels launched with programmatic
+/// stream serialization: coherent, and volatile so that the compiler keeps them behind `griddepcontrol.wait`. A
+/// read-only load (`__ldg`) is neither: the compiler may move it in front of the wait, and did (a GEMV over 2560
+/// columns read its activations before the norm that wrote them had run).
+__device__ __forceinline__ uint4 ld_after_wait16(const void *p)
+{
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint2 ld_after_wait8(const void *p)
+{
+    uint2 v;
+    asm volatile("ld.global.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+    return v;
+}
+
 /// The two bf16 halves of a word, widened (a bf16 is the top half of an f32).
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }

@@ -132,7 +132,7 @@ __device__ __forceinline__ void load_x32(const uint16_t *x, size_t off, bool liv
     const uint4 *xp = reinterpret_cast<const uint4 *>(x + off);
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
-        const uint4 xv = live ? __ldg(xp + v) : make_uint4(0, 0, 0, 0);
+        const uint4 xv = live ? dev::ld_after_wait16(xp + v) : make_uint4(0, 0, 0, 0);
         xr[4 * v] = xv.x, xr[4 * v + 1] = xv.y, xr[4 * v + 2] = xv.z, xr[4 * v + 3] = xv.w;
     }
 }

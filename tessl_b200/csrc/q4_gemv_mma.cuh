@@ -635,10 +635,10 @@ __global__ void __launch_bounds__(kThreads, TESSL_GEMV_MMA_MIN_BLOCKS) q4_gemv_m
                     for (int u = 0; u < WPG; ++u) {
                         const uint32_t k = k0 + jj * G + t * (G / 4) + 8 * u;
                         if constexpr (Q8) {
-                            const uint2 r = __ldg(reinterpret_cast<const uint2 *>(xrow + k / 2));
+                            const uint2 r = dev::ld_after_wait8(xrow + k / 2);
                             amax = max(amax, max(max(r.x & 0x7fffu, (r.x >> 16) & 0x7fffu), max(r.y & 0x7fffu, (r.y >> 16) & 0x7fffu)));
                         } else {
-                            const uint4 r = __ldg(reinterpret_cast<const uint4 *>(xrow + k));
+                            const uint4 r = dev::ld_after_wait16(xrow + k);
                             amax = max(amax, max(max(r.x & 0x7fffu, (r.x >> 16) & 0x7fffu), max(r.y & 0x7fffu, (r.y >> 16) & 0x7fffu)));
                             amax = max(amax, max(max(r.z & 0x7fffu, (r.z >> 16) & 0x7fffu), max(r.w & 0x7fffu, (r.w >> 16) & 0x7fffu)));
                         }
@@ -713,12 +713,12 @@ __global__ void __launch_bounds__(kThreads, TESSL_GEMV_MMA_MIN_BLOCKS) q4_gemv_m
                         // the word holds 4 codes; a code 0..255 read as a bf16 bit pattern is c * 2^-133 exactly (the
                         // subnormals and the first binade form one linear scale), so (w & 0x00ff00ff) is an A register
                         // of codes 0, 2 and ((w >> 8) & 0x00ff00ff) one of codes 1, 3: no magic constant, no offset
-                        const uint2 r = __ldg(reinterpret_cast<const uint2 *>(xrow + k / 2));
+                        const uint2 r = dev::ld_after_wait8(xrow + k / 2);
                         xb[jj * WPG + u][0] = pair(r.x, r.y, e);              // x0, x2
                         xb[jj * WPG + u][1] = pair(r.x >> 16, r.y >> 16, e);  // x1, x3
                         part += (dev::bf16_lo(r.x) + dev::bf16_hi(r.x)) + (dev::bf16_lo(r.y) + dev::bf16_hi(r.y));
                     } else {
-                        const uint4 r = __ldg(reinterpret_cast<const uint4 *>(xrow + k));
+                        const uint4 r = dev::ld_after_wait16(xrow + k);
                         xb[jj * WPG + u][0] = pair(r.x, r.z, e);                  // x0, x4
                         xb[jj * WPG + u][1] = pair(r.x >> 16, r.z >> 16, e - 4);  // (x1, x5) / 16
                         xb[jj * WPG + u][2] = pair(r.y, r.w, e);                  // x2, x6

@@ -207,3 +207,46 @@ def test_an_mlp_block_is_three_launches_and_replays_from_a_graph(rt):
             assert np.array_equal(resid.read(np.uint32, hidden), got.view(np.uint32))
     finally:
         rt.set_encode_only(False)
+
+
+@pytest.mark.parametrize("m,cols", [(1, 2560), (1, 544), (1, 4096), (4, 2048), (1, 9216)])
+def test_a_projection_reads_what_the_norm_before_it_wrote(rt, m, cols):
+    """Launches back to back in a CUDA graph (each may start before the one in front of it ends) that rewrite the same
+    activation buffer: every projection sees the norm in front of it and not an earlier one, bit for bit what it
+    gives when every call is waited for. 544 columns run on the kernel without bulk copies (17 groups of 32)."""
+    import torch
+
+    rows, group, steps = 640, 32 if cols == 544 else 64, 6
+    bank = upload_bank(rt, *synth.q4_bank(0x7E550B00, rows, cols, group))
+    shape = nn.QuantShape(rows, cols, group)
+    xs = [rt.buffer_from(synth.bf16_bits_to_f32(synth.normal_bf16(0x7E550B10 + i, m * cols))) for i in range(steps)]
+    w = rt.buffer_from(synth.bf16_bits_to_f32(synth.normal_bf16(0x7E550B30, cols)))
+    xb = rt.alloc_buffer(m * cols * 2)
+    ys = [rt.alloc_buffer(m * rows * 4) for _ in range(steps)]
+
+    def chain():
+        for x, y in zip(xs, ys):
+            nn.qwen35_rms_norm(rt, x, w, xb, True, m, cols, 1e-6)
+            if m == 1:
+                nn.gemv_q4_mlx_simd(rt, bank, xb, y, shape)
+            else:
+                nn.gemm_q4_mlx(rt, bank, xb, y, shape, m)
+
+    chain()
+    want = [y.read(np.uint32, m * rows) for y in ys]
+    st = torch.cuda.ExternalStream(rt.stream)
+    rt.set_encode_only(True)
+    try:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=st):
+            chain()
+        for y in ys:
+            y.write(np.zeros(m * rows, np.uint32))
+        with torch.cuda.stream(st):
+            for _ in range(3):
+                graph.replay()
+        rt.synchronize()
+    finally:
+        rt.set_encode_only(False)
+    for i, (y, v) in enumerate(zip(ys, want)):
+        assert np.array_equal(y.read(np.uint32, m * rows), v), f"step {i}"
