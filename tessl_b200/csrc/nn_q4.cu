@@ -3,17 +3,20 @@
 // the reference project): validation in the reference's order and wording, the choice of kernel and
 // instantiation, the launch.
 //
-// Kernels: q4_gemv_mma.cuh (the default: dot products on the tensor cores, bulk-copy ring; also the MLX Q8 mode
-// and the column-sharded launches that exchange their outputs over NVLink), and the FMA-pipe fallbacks
-// q4_gemv_tma.cuh, q4_gemv_warp.cuh, q4_gemv_main.cuh / q4_gemv_kernel.cuh for the shapes it does not take.
+// Kernels: q4_gemv_mma.cuh (one row of x at the common widths: dot products on the tensor cores, bulk-copy ring; also
+// the MLX Q8 mode and the column-sharded launches that exchange their outputs over NVLink), q4_batch_mma.cuh (2..8 rows,
+// and one row at the other widths: the same arithmetic, any whole number of 256-column chunks), and the FMA-pipe
+// fallbacks q4_gemv_tma.cuh, q4_gemv_warp.cuh, q4_gemv_main.cuh / q4_gemv_kernel.cuh for the shapes these do not take.
 #include "q4_gemv_main.cuh"
 #include "q4_gemv_warp.cuh"
 #include "q4_gemv_tma.cuh"
 #include "q4_gemv_mma.cuh"
+#include "q4_batch_mma.cuh"
 
 #include <cstdio>
 #include <cstdlib>
 #include "runtime.h"
+#include "tensormap.h"
 
 namespace tessl {
 namespace {
@@ -285,19 +288,12 @@ bool mma_ok(const Q4GemvParams &p)
     return true;
 }
 
-/// A launch over a window of `cols` columns of longer rows (one K chunk): distances in global
-/// memory between packed rows and scale/bias rows (bytes) and between batch rows of x (elements).
-/// Zeros: dense rows.
-struct MmaWindow {
-    uint32_t row_pitch = 0, sb_pitch = 0, x_pitch = 0;
-};
-
 /// Shared memory one block of the tensor-core GEMV may use: the per-block maximum of sm_100 less the kernel's few
 /// static bytes.
 constexpr uint32_t kMmaSmemBudget = 232448u - 512u;
 
 template <int SW, int WPG, int NB, bool BATCH, bool Q8 = false, int NWIN = 1, int ROWS = 16, bool STAGED = false>
-Result launch_mma_one(TesslRuntime *rt, const Q4GemvParams &p, int m, const MmaWindow &w = MmaWindow{})
+Result launch_mma_one(TesslRuntime *rt, const Q4GemvParams &p, int m)
 {
     auto kernel = q4m::q4_gemv_mma_kernel<SW, WPG, NB, BATCH, Q8, NWIN, ROWS, STAGED>;
     constexpr uint32_t RPB = ROWS / NB;
@@ -312,9 +308,6 @@ Result launch_mma_one(TesslRuntime *rt, const Q4GemvParams &p, int m, const MmaW
     mp.nseg = p.nseg, mp.total_rb = rb;
     mp.x = p.x, mp.m = (uint32_t)m, mp.cols = p.cols, mp.group_shift = p.group_shift;
     mp.epi = p.epi, mp.out_bf16 = p.out_bf16;
-    mp.row_pitch = w.row_pitch ? w.row_pitch : p.cols >> 1;
-    mp.sb_pitch = w.sb_pitch ? w.sb_pitch : (p.cols >> p.group_shift) * 4;
-    mp.x_pitch = w.x_pitch ? w.x_pitch : (Q8 ? p.cols >> 1 : p.cols);
     mp.status = rt->status_dev;
     if ((p.staged != 0) != STAGED) return "q4_gemv: the staged layout runs on the one-row Q4 kernel only";
     if (p.peer) {
@@ -353,7 +346,7 @@ Result launch_mma_one(TesslRuntime *rt, const Q4GemvParams &p, int m, const MmaW
     // four rows per bulk copy wherever two row pairs are adjacent in memory (one bank, dense rows): 151936 x 4096
     // 58.8 -> 52.7 us, 6144 x 4096 5.30 -> 5.05 us, 12288 x 4096 8.00 -> 7.90 us on one box, back to back.
     // Not for Q8: its row pair is already 8 KB, and 16 KB copies ran 14336 x 4096 in 17.0 us against 14.5.
-    mp.quads = (!BATCH && !Q8 && NWIN == 1 && w.row_pitch == 0 && !p.staged) ? 1u : 0u;
+    mp.quads = (!BATCH && !Q8 && NWIN == 1 && !p.staged) ? 1u : 0u;
     cudaLaunchConfig_t lc{};
     lc.gridDim = dim3(grid), lc.blockDim = dim3(q4m::kThreads), lc.dynamicSmemBytes = smem;
     lc.stream = rt->stream;
@@ -367,33 +360,32 @@ Result launch_mma_one(TesslRuntime *rt, const Q4GemvParams &p, int m, const MmaW
 }
 
 template <int SW, int WPG>
-Result launch_mma_sw(TesslRuntime *rt, const Q4GemvParams &p, int m, int nb, const MmaWindow &w)
+Result launch_mma_sw(TesslRuntime *rt, const Q4GemvParams &p, int nb)
 {
     if (p.staged) {
-        if (m != 1 || w.row_pitch != 0) return "q4_gemv: the staged layout runs on the one-row Q4 kernel only";
-        if (nb == 2) return launch_mma_one<SW, WPG, 2, false, false, 1, 16, true>(rt, p, m, w);
-        return launch_mma_one<SW, WPG, 1, false, false, 1, 16, true>(rt, p, m, w);
+        if (nb == 2) return launch_mma_one<SW, WPG, 2, false, false, 1, 16, true>(rt, p, 1);
+        return launch_mma_one<SW, WPG, 1, false, false, 1, 16, true>(rt, p, 1);
     }
-    if (nb == 2) return launch_mma_one<SW, WPG, 2, false>(rt, p, m, w);
-    if (m == 1) return launch_mma_one<SW, WPG, 1, false>(rt, p, m, w);
-    return launch_mma_one<SW, WPG, 1, true>(rt, p, m, w);
+    if (nb == 2) return launch_mma_one<SW, WPG, 2, false>(rt, p, 1);
+    return launch_mma_one<SW, WPG, 1, false>(rt, p, 1);
 }
 
-Result launch_mma(TesslRuntime *rt, const Q4GemvParams &p, int m, int nb, const MmaWindow &w = MmaWindow{})
+/// One row of x.
+Result launch_mma(TesslRuntime *rt, const Q4GemvParams &p, int nb)
 {
     const int sw = (int)(p.cols / 512), wpg = 1 << (p.group_shift - 5);
     if (sw == 8) {
-        if (wpg == 1) return launch_mma_sw<8, 1>(rt, p, m, nb, w);
-        if (wpg == 2) return launch_mma_sw<8, 2>(rt, p, m, nb, w);
-        return launch_mma_sw<8, 4>(rt, p, m, nb, w);
+        if (wpg == 1) return launch_mma_sw<8, 1>(rt, p, nb);
+        if (wpg == 2) return launch_mma_sw<8, 2>(rt, p, nb);
+        return launch_mma_sw<8, 4>(rt, p, nb);
     }
     if (sw == 4) {
-        if (wpg == 1) return launch_mma_sw<4, 1>(rt, p, m, nb, w);
-        if (wpg == 2) return launch_mma_sw<4, 2>(rt, p, m, nb, w);
-        return launch_mma_sw<4, 4>(rt, p, m, nb, w);
+        if (wpg == 1) return launch_mma_sw<4, 1>(rt, p, nb);
+        if (wpg == 2) return launch_mma_sw<4, 2>(rt, p, nb);
+        return launch_mma_sw<4, 4>(rt, p, nb);
     }
-    if (wpg == 1) return launch_mma_sw<2, 1>(rt, p, m, nb, w);
-    return launch_mma_sw<2, 2>(rt, p, m, nb, w);
+    if (wpg == 1) return launch_mma_sw<2, 1>(rt, p, nb);
+    return launch_mma_sw<2, 2>(rt, p, nb);
 }
 
 /// One row of x over rows of 8192 or 12288 columns (a 4096 x 12288 down projection): the tensor-core kernel
@@ -425,31 +417,141 @@ Result launch_mma_long(TesslRuntime *rt, const Q4GemvParams &p)
     return launch_mma_one<8, 4, 1, false, false, 3, 14>(rt, p, 1);
 }
 
-/// Batches of 3..8 rows over rows longer than the tensor-core kernel's 4096 columns (a 12288-column
-/// down projection in batched decode): one launch of that kernel per window of 4096 columns, each
-/// after the first adding to the f32 result of those before it (the kernel's add-residual epilogue
-/// with the output as the residual; launches on one stream are ordered). The FMA-pipe kernel this
-/// replaces costs one pass per batch row (4096 x 12288: 65 us at M = 8 against 21 us here; at
-/// M = 2 it is still the faster one, 17 us against 20 us). Returns false if the call does not fit.
-bool launch_mma_windows(TesslRuntime *rt, const Q4GemvParams &p, int m, int nb, Result &res)
+/// How the batch kernel (q4_batch_mma.cuh) cuts a row: windows of whole units, each window's groups dealt out to the
+/// 16 consumer warps. `ngs` is the busiest warp's share; 0 if the kernel does not take the shape.
+struct BatchPlan {
+    uint32_t unit_cols = 0, units = 0, nwin = 0, chunks = 0, sb_boxes = 0;
+    int ngs = 0;
+    bool even = false;  // every warp has ngs groups in every window, and ngs is a power of two
+};
+BatchPlan batch_plan(uint32_t cols, uint32_t group_shift)
 {
-    constexpr uint32_t W = 4096;
-    if (m < 3 || m > 8 || nb != 1 || p.nseg != 1 || p.cols <= W || p.cols % W != 0 || p.out_bf16) return false;
-    if (p.epi != q4k::EPI_STORE) return false;  // a residual is added once, after the whole sum: not expressible here
-    Q4GemvParams q = p;
-    q.cols = W;
-    if (!mma_ok(q)) return false;
-    MmaWindow w;
-    w.row_pitch = p.cols >> 1, w.sb_pitch = (p.cols >> p.group_shift) * 4, w.x_pitch = p.cols;
-    for (uint32_t c = 0; c < p.cols / W; ++c) {
-        q.x = p.x + (size_t)c * W;
-        q.seg[0].packed0 = p.seg[0].packed0 + (size_t)c * (W / 2);
-        q.seg[0].sb0 = p.seg[0].sb0 + (size_t)c * (W >> p.group_shift);
-        if (c > 0) q.epi = q4k::EPI_ADD_RESID, q.seg[0].resid = static_cast<const float *>(p.seg[0].out);
-        res = launch_mma(rt, q, m, 1, w);
-        if (!res.empty()) return true;
+    BatchPlan b;
+    if (group_shift < 5 || group_shift > 7 || cols == 0) return b;
+    // a window starts on a whole 256-column chunk of the packed rows and a whole quad of groups (16 bytes of pairs)
+    b.unit_cols = std::max<uint32_t>(q4b::kChunkCols, 4u << group_shift);
+    if (cols % b.unit_cols != 0) return b;
+    b.units = cols / b.unit_cols;
+    const uint32_t per = q4b::kWindowCols / b.unit_cols;
+    b.nwin = (b.units + per - 1) / per;
+    // Four windows instead of three: clusters of three leave 13 SMs without one and start late (4096 x 8192 at M = 8 cut in
+    // 2 / 3 / 4: 7.4 / 11.3 / 7.2 us; 4096 x 12288 in 3 / 4: 10.4 / 8.9 us).
+    if (b.nwin == 3) b.nwin = 4;
+    if (b.nwin > q4b::kMaxWindows) return b;
+    uint32_t widest = 0, narrowest = ~0u;
+    for (uint32_t c = 0; c < b.nwin; ++c) {
+        const uint32_t n = (c + 1) * b.units / b.nwin - c * b.units / b.nwin;
+        widest = std::max(widest, n), narrowest = std::min(narrowest, n);
     }
-    return true;
+    const uint32_t gpu = b.unit_cols >> group_shift;  // groups per unit
+    b.chunks = widest * (b.unit_cols / q4b::kChunkCols);
+    b.sb_boxes = (widest * gpu + 31) / 32;
+    const int ngs = (int)((widest * gpu + q4b::kConsumers - 1) / q4b::kConsumers);
+    if ((int)(narrowest * gpu / q4b::kConsumers) < ngs - 1) return b;  // warps hold ngs or ngs - 1 groups in every window
+    b.ngs = ngs;
+    b.even = narrowest == widest && widest * gpu == (uint32_t)ngs * q4b::kConsumers && (ngs & (ngs - 1)) == 0;
+    return b;
+}
+
+bool batch_ok(const Q4GemvParams &p, int m, int nb)
+{
+    if (!mma_enabled() || m < 1 || m > 8 || (nb != 1 && m != 1) || p.staged || p.peer || p.xwait) return false;
+    for (int s = 0; s < p.nseg; ++s) {
+        const Q4Seg &a = p.seg[s];
+        if (((uintptr_t)a.sb0 | (uintptr_t)a.packed0 | (uintptr_t)a.sb1 | (uintptr_t)a.packed1) & 15u) return false;
+    }
+    return batch_plan(p.cols, p.group_shift).ngs != 0;
+}
+
+template <int WPG, int NGS, bool EVEN, int NB>
+Result launch_batch_one(TesslRuntime *rt, const Q4GemvParams &p, int m, const BatchPlan &b)
+{
+    auto kernel = q4b::q4_batch_mma_kernel<WPG, NGS, EVEN, NB>;
+    constexpr uint32_t RPB = q4b::kRows / NB;
+    const char *what = "q4_gemv";
+    EncodeTiled enc = nullptr;
+    TESSL_TRY(tensormap_encoder(rt, what, &enc));
+    q4b::Maps maps;
+    q4b::Params bp{};
+    const uint32_t gpr = p.cols >> p.group_shift;
+    auto encode = [&](int i, const uint8_t *packed, const uint32_t *sb, uint32_t rows) -> Result {
+        const cuuint64_t dims[3] = {128, rows, p.cols / q4b::kChunkCols}, strides[2] = {p.cols / 2, 128};
+        const cuuint32_t box[3] = {128, RPB, b.chunks};
+        TESSL_TRY(make_map(enc, what, &maps.w[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, packed, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B));
+        const cuuint64_t sdims[2] = {gpr, rows}, sstrides[1] = {(cuuint64_t)gpr * 4};
+        const cuuint32_t sbox[2] = {32, RPB};
+        return make_map(enc, what, &maps.sb[i], CU_TENSOR_MAP_DATA_TYPE_UINT32, sb, sdims, sstrides, sbox, CU_TENSOR_MAP_SWIZZLE_128B);
+    };
+    for (int s = 0; s < p.nseg; ++s) {
+        const Q4Seg &a = p.seg[s];
+        if (a.rows == 0) return fmt("%s: a bank with no rows takes no part in a launch", what);
+        TESSL_TRY(encode(s, a.packed0, a.sb0, a.rows));
+        if (NB == 2) TESSL_TRY(encode(1, a.packed1, a.sb1, a.rows));
+        bp.seg[s] = q4b::Seg{a.out, a.resid, a.rows, bp.total_rb};
+        bp.total_rb += (uint32_t)(((uint64_t)a.rows + RPB - 1) / RPB);
+    }
+    bp.x = p.x, bp.status = rt->status_dev;
+    bp.nseg = (uint32_t)p.nseg, bp.cols = p.cols, bp.m = (uint32_t)m, bp.group_shift = p.group_shift;
+    bp.units = b.units, bp.unit_cols = b.unit_cols, bp.nwin = b.nwin, bp.chunks = b.chunks, bp.sb_boxes = b.sb_boxes;
+    bp.epi = p.epi, bp.out_bf16 = p.out_bf16;
+    const uint32_t stage_bytes = (b.chunks + b.sb_boxes) * q4b::kBoxBytes + q4b::kPartBytes;
+    const uint32_t fixed = 1024 + q4b::kMailSlots * (b.nwin - 1) * q4b::kMailBytes + 8 * (1 + 2 * q4b::kMailSlots);
+    bp.stages = std::min<uint32_t>(8u, (kMmaSmemBudget - fixed) / (stage_bytes + 24));
+    if (bp.stages < (uint32_t)q4b::kReducers) return "q4_batch_mma: the ring does not fit two stages";
+    const size_t smem = fixed + (size_t)bp.stages * (stage_bytes + 24);
+    TESSL_TRY(smem_opt_in(rt, reinterpret_cast<const void *>(kernel), smem, "q4_batch_mma: shared memory opt-in", true));
+
+    cudaLaunchConfig_t lc{};
+    lc.blockDim = dim3(q4b::kThreads), lc.dynamicSmemBytes = smem;
+    lc.stream = rt->stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = b.nwin, attr[1].val.clusterDim.y = 1, attr[1].val.clusterDim.z = 1;
+    lc.attrs = attr, lc.numAttrs = b.nwin > 1 ? 2 : 1;
+    uint32_t clusters = (uint32_t)rt->sm_count;
+    if (b.nwin > 1) {
+        // how many clusters of this size the device holds at once (one CTA per SM; a cluster lies in one GPC)
+        int &n = rt->max_clusters[std::make_pair(reinterpret_cast<const void *>(kernel), b.nwin)];
+        if (n == 0) {
+            lc.gridDim = dim3(b.nwin * (rt->sm_count / b.nwin));
+            const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, kernel, &lc);
+            if (e != cudaSuccess || n < 1) {
+                cudaGetLastError();
+                n = std::max(1, rt->sm_count / (int)b.nwin);
+            }
+        }
+        clusters = (uint32_t)n; 
+    }
+    clusters = std::min(clusters, bp.total_rb);
+    const uint64_t step = (((uint64_t)bp.total_rb << 32) + clusters - 1) / clusters;
+    bp.rb_step_lo = (uint32_t)step, bp.rb_step_hi = (uint32_t)(step >> 32);
+    lc.gridDim = dim3(clusters * b.nwin);
+    const cudaError_t e = cudaLaunchKernelEx(&lc, kernel, maps, bp);
+    rt->dispatch_count += 1;
+    return cuda_check(rt, e, "q4_gemv launch");
+}
+
+template <int WPG, int NGS>
+Result launch_batch_ngs(TesslRuntime *rt, const Q4GemvParams &p, int m, int nb, const BatchPlan &b)
+{
+    if constexpr (NGS > 1) {
+        if (b.ngs != NGS) return launch_batch_ngs<WPG, NGS - 1>(rt, p, m, nb, b);
+    }
+    if (nb == 2) return launch_batch_one<WPG, NGS, false, 2>(rt, p, m, b);
+    if constexpr ((NGS & (NGS - 1)) == 0) {
+        if (b.even) return launch_batch_one<WPG, NGS, true, 1>(rt, p, m, b);
+    }
+    return launch_batch_one<WPG, NGS, false, 1>(rt, p, m, b);
+}
+
+Result launch_batch(TesslRuntime *rt, const Q4GemvParams &p, int m, int nb)
+{
+    const BatchPlan b = batch_plan(p.cols, p.group_shift);
+    if (p.group_shift == 5) return launch_batch_ngs<1, 8>(rt, p, m, nb, b);
+    if (p.group_shift == 6) return launch_batch_ngs<2, 4>(rt, p, m, nb, b);
+    return launch_batch_ngs<4, 2>(rt, p, m, nb, b);
 }
 
 template <int SW, int WPG>
@@ -512,7 +614,8 @@ Result launch_q4_gemv(TesslRuntime *rt, Q4GemvParams p, int m, int nb)
     const uint32_t nchunks = std::max<uint32_t>(1u, (p.cols + q4k::kChunk - 1) / q4k::kChunk);
     if (p.staged && !(m == 1 && mma_ok(p)))
         return "q4_gemv: the staged layout needs the tensor-core GEMV kernel (one row of x, rows of 1024, 2048 or 4096 columns)";
-    if (m >= 1 && m <= 8 && (nb == 1 || m == 1) && mma_ok(p)) return launch_mma(rt, p, m, nb);
+    if (m > 1 && batch_ok(p, m, nb)) return launch_batch(rt, p, m, nb);
+    if (m == 1 && mma_ok(p)) return launch_mma(rt, p, nb);
     if (mma_long_ok(p, m)) {
         // The kernel takes one bank per launch at these widths. The bank-routed forms run as one launch per
         // bank, the gate/up forms as two launches into scratch and the activation kernel: what the fused
@@ -542,10 +645,11 @@ Result launch_q4_gemv(TesslRuntime *rt, Q4GemvParams p, int m, int nb)
         if (p.peer) return nn::peer_gather(rt, *static_cast<const TesslPeerGather *>(p.peer));
         return ok();
     }
-    {
-        Result res = ok();
-        if (launch_mma_windows(rt, p, m, nb, res)) return res;
-    }
+    // One row of x over shorter rows leaves most of the 16 consumer warps without a group: 60000 x 512 8.9 us on the FMA
+    // pipe against 12.5 here, 4096 x 512 2.33 / 2.48; from 1024 columns on 1024 x 1280 2.61 / 2.27, 6144 x 2560 5.50 / 4.26,
+    // 2048 x 6144 4.72 / 4.85, 2560 x 9216 7.55 / 6.70, 4096 x 17408 24.6 / 12.3, 40000 x 6144 35.4 / 26.2. A function of K
+    // alone, so that a row's summation order stays one of K and G.
+    if (m == 1 && p.cols >= 1024 && batch_ok(p, m, nb)) return launch_batch(rt, p, m, nb);
     if (m == 1 && nchunks <= 4 && tma_ok(p)) {
         if (nb == 1) {
             if (nchunks == 1) return launch_tma<1, 8, 1>(rt, p);

@@ -49,6 +49,7 @@
 
 #include "prefill_common.cuh"
 #include "prefill_gemm_pair.cuh"
+#include "tensormap.h"
 
 namespace tessl {
 namespace {
@@ -382,37 +383,14 @@ __global__ void __launch_bounds__(Cfg<BN>::THREADS, 1)
 
 // ---------------------------------------------------------------------- host ---
 
-using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                 const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-Result tensormap_encoder(TesslRuntime *rt, EncodeTiled *out)
-{
-    if (!rt->tensormap_encode) {
-        void *fn = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q);
-        if (e != cudaSuccess || q != cudaDriverEntryPointSuccess || !fn) {
-            cudaGetLastError();
-            return "gemm_q4_mlx_tensorops: the driver does not export cuTensorMapEncodeTiled";
-        }
-        rt->tensormap_encode = fn;
-    }
-    *out = reinterpret_cast<EncodeTiled>(rt->tensormap_encode);
-    return ok();
-}
+constexpr const char *kWhat = "gemm_q4_mlx_tensorops";
 
 Result make_map_2d(EncodeTiled enc, CUtensorMap *map, CUtensorMapDataType dt, void *ptr, uint64_t inner, uint64_t outer,
                    uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer, CUtensorMapSwizzle swz)
 {
-    const cuuint64_t dims[2] = {inner, outer};
-    const cuuint64_t strides[1] = {row_stride_bytes};
+    const cuuint64_t dims[2] = {inner, outer}, strides[1] = {row_stride_bytes};
     const cuuint32_t box[2] = {box_inner, box_outer};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = enc(map, dt, 2, ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fmt("gemm_q4_mlx_tensorops: cuTensorMapEncodeTiled failed (%d)", (int)r);
-    return ok();
+    return make_map(enc, kWhat, map, dt, ptr, dims, strides, box, swz);
 }
 
 template <int BN>
@@ -535,7 +513,7 @@ Result prefill_launch(TesslRuntime *rt, const TesslQ4MlxBank &bank, const TesslB
     rt->prefill_last_bn = bn, rt->prefill_last_pair = pair ? 1 : 0;
 
     EncodeTiled enc = nullptr;
-    TESSL_TRY(tensormap_encoder(rt, &enc));
+    TESSL_TRY(tensormap_encoder(rt, kWhat, &enc));
     CUtensorMap ma, mw;
     TESSL_TRY(make_map_2d(enc, &ma, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a_aug, pl.k_aug, m, (uint64_t)pl.k_aug * 2, BK, BM,
                           CU_TENSOR_MAP_SWIZZLE_128B));

@@ -49,6 +49,34 @@ __device__ __forceinline__ uint2 ld_after_wait8(const void *p)
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 
+/// Power-of-two scaling of a slice of bf16 activations that meets nibbles held as bf16 subnormals (q * 2^-133): `mul` =
+/// (2^e, 2^e) and `mul16` = (2^(e-4), 2^(e-4)) as bf16 pairs, `undo` = 2^(133-e). e brings the slice's largest magnitude
+/// to about 2^100, so that every product is a normal f32, within what a bf16 factor (e <= 127) and an f32 undo (e >= 6)
+/// can hold. `amax`: the largest magnitude's bits; a slice of zeros and subnormals counts as zero.
+struct XScale {
+    uint32_t mul, mul16;
+    float undo;
+};
+__device__ __forceinline__ XScale x_scale(uint32_t amax)
+{
+    if ((amax >> 7) == 0) return XScale{0u, 0u, 0.0f};
+    const int e = min(127, max(6, 100 + 127 - (int)(amax >> 7)));
+    return XScale{(uint32_t)(e + 127) * 0x00800080u, (uint32_t)(e + 123) * 0x00800080u, __uint_as_float((uint32_t)(127 + 133 - e) << 23)};
+}
+__device__ __forceinline__ uint32_t bf2_mul(uint32_t a, uint32_t b)
+{
+    uint32_t r;
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+/// Eight activations -> the B registers of the two MMAs that take the eight nibbles of a packed word:
+/// (x0, x4), (x1, x5) / 16, (x2, x6), (x3, x7) / 16, scaled. Exact: only exponents change.
+__device__ __forceinline__ void x_fragment(const uint4 &v, const XScale &s, uint32_t (&f)[4])
+{
+    f[0] = bf2_mul(__byte_perm(v.x, v.z, 0x5410), s.mul), f[1] = bf2_mul(__byte_perm(v.x, v.z, 0x7632), s.mul16);
+    f[2] = bf2_mul(__byte_perm(v.y, v.w, 0x5410), s.mul), f[3] = bf2_mul(__byte_perm(v.y, v.w, 0x7632), s.mul16);
+}
+
 /// f32 -> bf16 bits as the reference's device cast stores them
 /// (`f32_to_bf16_bits_gpu`, src/tensor.rs:815-831 of the reference project):
 /// any NaN becomes 0x7fc0, an f32 subnormal flushes to a zero of its sign,

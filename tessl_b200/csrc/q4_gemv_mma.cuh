@@ -1,5 +1,5 @@
-// Q4 GEMV / small-batch GEMM (M <= 8, rows of 1024, 2048 or 4096 columns; one row of x also over rows of 8192 and
-// 12288 columns) and MLX-layout Q8 (M <= 8), with the dot products on the tensor cores.
+// Q4 GEMV (one row of x; rows of 1024, 2048, 4096, 8192 or 12288 columns) and MLX-layout Q8 (M <= 8), with the dot
+// products on the tensor cores. Q4 batches and the other widths: q4_batch_mma.cuh, with the same arithmetic.
 //
 // Why: on the FMA pipe a weight costs one FMA plus 7/8 of a bit-manipulation
 // instruction plus overheads, about 2 issue slots; HBM3e delivers ~46 weights
@@ -11,7 +11,7 @@
 // the first binade are one linear scale), and the activations carry the rest
 // (scaled by a power of two, the partners of the odd nibbles by a sixteenth of it).
 // So one MMA replaces 256 FMAs: 16 weight rows x 16 columns against the
-// activations as the B operand, whose 8 columns are the up to 8 rows of the batch
+// activations as the B operand, whose 8 columns are the up to 8 rows of a Q8 batch
 // (for M = 1 all 8 hold the same vector). The kernel is then bound by the weight
 // stream on a long launch and by its start and the consumers' ALU rate on a short one.
 //
@@ -113,12 +113,6 @@ struct Params {
     uint32_t m;
     int epi;
     int out_bf16;
-    // A launch may cover a window of `cols` columns of longer rows (a K chunk): bytes between packed
-    // rows and between scale/bias rows in global memory, elements between the batch rows of x. Dense
-    // rows: cols / 2, (cols >> group_shift) * 4 and cols.
-    uint32_t row_pitch;
-    uint32_t sb_pitch;
-    uint32_t x_pitch;
     uint32_t quads;  // fetch four rows per bulk copy (long streams, one bank, one row of x)
     // Row blocks per thread block as a 32.32 fixed-point number, rounded up: block b takes the row blocks
     // [b step >> 32, (b + 1) step >> 32) clipped to total_rb. (The division total_rb b / blocks in the kernel is a
@@ -126,15 +120,15 @@ struct Params {
     uint32_t rb_step_lo, rb_step_hi;
     uint32_t peer_world;   // == peer.world
     uint32_t xwait_world;  // == xwait.world
-    // --- line 1: the activations and the first bank
     const uint16_t *x;  // bf16 [m, cols]
+    // --- line 1: the first bank
     Seg seg[3];
     // --- cold: failure reports and the exchange
     uint32_t *status;
     Peer peer;
     XWait xwait;
 };
-static_assert(offsetof(Params, x) == 64 && offsetof(Params, seg) == 72 && sizeof(Seg) == 56, "parameter lines");
+static_assert(offsetof(Params, x) == 56 && offsetof(Params, seg) == 64 && sizeof(Seg) == 56, "parameter lines");
 
 // A system-scope fence, and every acquire or release at system scope, costs ~1.8 us on this GPU (measured: the
 // same for local and for peer stores). The exchange therefore polls and signals with RELAXED system-scope
@@ -210,8 +204,8 @@ __global__ void __launch_bounds__(kThreads, TESSL_GEMV_MMA_MIN_BLOCKS) q4_gemv_m
     static_assert(ROWS % (2 * NB) == 0 && ROWS <= 16, "whole row pairs per bank");
     constexpr int NGS = SW / WPG;     // groups per slice
     constexpr int RPB = ROWS / NB;    // rows per bank and stage
-    constexpr int NQ = (NGS + 3) / 4;  // affine groups per lane when M = 1
-    static_assert(SW % WPG == 0 && NGS >= 1, "a warp's slice holds whole groups");
+    static_assert(SW % WPG == 0 && (NGS == 1 || NGS == 2 || NGS % 4 == 0), "a warp's slice holds whole groups");
+    static_assert(!BATCH || Q8, "Q4 batches run on q4_batch_mma.cuh");
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ int abort_flag;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -297,17 +291,13 @@ __global__ void __launch_bounds__(kThreads, TESSL_GEMV_MMA_MIN_BLOCKS) q4_gemv_m
         // instructions per stage: the warp shares its scheduler with consumer warps that
         // saturate it, so every instruction here waits for an issue slot. Lanes 0-15 own
         // the 16 row slots of a stage, lanes 16 (and 17) the scale/bias rows of a bank.
-        // Windowed rows (NB = 1 only): the scale/bias rows are not contiguous, lanes 16-31 fetch one each.
-        const bool sb_by_row = NB == 1 && p.sb_pitch != sb_row_bytes;
-        const bool pair_copy = p.row_pitch == row_bytes;  // dense rows: two adjacent rows are one contiguous range
         constexpr uint32_t HP = RPB / 2;                  // row pairs per bank and stage
         // lane m < 16 owns MMA row m: lane group g = m % 8, upper half hi = m / 8 -> bank g / HP, local row 2 (g % HP) + hi
         const uint32_t mg = (uint32_t)lane & 7u, mhi = ((uint32_t)lane >> 3) & 1u;
-        const uint32_t my_bank = lane < 16 ? mg / HP : (sb_by_row ? 0u : (uint32_t)lane - 16);
-        const uint32_t my_r = lane < 16 ? 2 * (mg % HP) + mhi : (sb_by_row ? (uint32_t)lane - 16 : 0u);
-        const bool copies = lane < 16 ? mg < HP * NB : (sb_by_row ? lane - 16 < RPB : lane < 16 + NB);
-        const uint32_t my_dst = lane < 16 ? pair_off(mg) + mhi * row_bytes
-                                          : off_sb + (sb_by_row ? my_r : my_bank * RPB) * sb_row_bytes;
+        const uint32_t my_bank = lane < 16 ? mg / HP : (uint32_t)lane - 16;
+        const uint32_t my_r = lane < 16 ? 2 * (mg % HP) + mhi : 0u;
+        const bool copies = lane < 16 ? mg < HP * NB : lane < 16 + NB;
+        const uint32_t my_dst = lane < 16 ? pair_off(mg) + mhi * row_bytes : off_sb + my_bank * RPB * sb_row_bytes;
         uint32_t s = 0, ph = 0, issued = 0;
         // the first stage that waits for x (see the loop); a block of exactly three stages holds its last one
         // (6144 x 4096: 4.64 -> 4.47 us)
@@ -329,12 +319,11 @@ __global__ void __launch_bounds__(kThreads, TESSL_GEMV_MMA_MIN_BLOCKS) q4_gemv_m
                 seg_end_rb = sg.rb_begin + (sg.rows + RPB - 1) / RPB;
                 row0 = (rb - sg.rb_begin) * RPB;
                 if (lane < 16) {
-                    src = (my_bank == 0 ? sg.packed0 : sg.packed1) + (size_t)(row0 + my_r) * p.row_pitch;
-                    src_step = RPB * p.row_pitch;
+                    src = (my_bank == 0 ? sg.packed0 : sg.packed1) + (size_t)(row0 + my_r) * row_bytes;
+                    src_step = RPB * row_bytes;
                 } else {
-                    src = reinterpret_cast<const uint8_t *>((my_bank == 0 ? sg.sb0 : sg.sb1)) +
-                          (size_t)(row0 + (sb_by_row ? my_r : 0u)) * p.sb_pitch;
-                    src_step = RPB * p.sb_pitch;
+                    src = reinterpret_cast<const uint8_t *>((my_bank == 0 ? sg.sb0 : sg.sb1)) + (size_t)row0 * sb_row_bytes;
+                    src_step = RPB * sb_row_bytes;
                 }
             }
             if (!mbar_wait(empty(s), ph ^ 1u, abortp, 64)) {
@@ -376,18 +365,11 @@ __global__ void __launch_bounds__(kThreads, TESSL_GEMV_MMA_MIN_BLOCKS) q4_gemv_m
             __syncwarp();
             if (copies) {
                 if (lane >= 16) {
-                    if (!sb_by_row) {
-                        bulk_g2s(st + my_dst, src, nrows * sb_row_bytes, full(s));
-                    } else if (my_r < nrows) {
-                        bulk_g2s(st + my_dst, src, sb_row_bytes, full(s));
-                    }
-                } else if (pair_copy) {
-                    if (quads && nrows == RPB) {
-                        if (mhi == 0 && (mg & 1u) == 0 && mg < HP * NB)
-                            bulk_g2s(st + my_dst, src, ((mg % HP) + 1 < HP ? 4 : 2) * row_bytes, full(s));
-                    } else if (mhi == 0 && my_r < nrows) bulk_g2s(st + my_dst, src, my_r + 1 < nrows ? 2 * row_bytes : row_bytes, full(s));
-                } else if (my_r < nrows) {
-                    bulk_g2s(st + my_dst, src, row_bytes, full(s));
+                    bulk_g2s(st + my_dst, src, nrows * sb_row_bytes, full(s));
+                } else if (quads && nrows == RPB) {
+                    if (mhi == 0 && (mg & 1u) == 0) bulk_g2s(st + my_dst, src, ((mg % HP) + 1 < HP ? 4 : 2) * row_bytes, full(s));
+                } else if (mhi == 0 && my_r < nrows) {
+                    bulk_g2s(st + my_dst, src, my_r + 1 < nrows ? 2 * row_bytes : row_bytes, full(s));
                 }
             }
             src += src_step, row0 += RPB;
@@ -625,39 +607,25 @@ __global__ void __launch_bounds__(kThreads, TESSL_GEMV_MMA_MIN_BLOCKS) q4_gemv_m
         };
         {
             const uint32_t n = BATCH ? min(g, p.m - 1) : 0u;
-            const uint16_t *xrow = p.x + (size_t)n * p.x_pitch;
-            int e = 0;
+            const uint16_t *xrow = p.x + (size_t)n * (Q8 ? K / 2 : K);
+            dev::XScale xsc{};
             if constexpr (BATCH || Q8) {
-                uint32_t amax = 0;
+                uint32_t amax2 = 0;  // two 16-bit maxima
 #pragma unroll
                 for (int jj = 0; jj < NGS; ++jj) {
 #pragma unroll
                     for (int u = 0; u < WPG; ++u) {
-                        const uint32_t k = k0 + jj * G + t * (G / 4) + 8 * u;
-                        if constexpr (Q8) {
-                            const uint2 r = dev::ld_after_wait8(xrow + k / 2);
-                            amax = max(amax, max(max(r.x & 0x7fffu, (r.x >> 16) & 0x7fffu), max(r.y & 0x7fffu, (r.y >> 16) & 0x7fffu)));
-                        } else {
-                            const uint4 r = dev::ld_after_wait16(xrow + k);
-                            amax = max(amax, max(max(r.x & 0x7fffu, (r.x >> 16) & 0x7fffu), max(r.y & 0x7fffu, (r.y >> 16) & 0x7fffu)));
-                            amax = max(amax, max(max(r.z & 0x7fffu, (r.z >> 16) & 0x7fffu), max(r.w & 0x7fffu, (r.w >> 16) & 0x7fffu)));
-                        }
+                        const uint2 r = dev::ld_after_wait8(xrow + (k0 + jj * G + t * (G / 4) + 8 * u) / 2);
+                        xb[jj * WPG + u][0] = r.x, xb[jj * WPG + u][1] = r.y;
+                        amax2 = __vmaxu2(amax2, __vmaxu2(r.x & 0x7fff7fffu, r.y & 0x7fff7fffu));
                     }
                 }
+                uint32_t amax = max(amax2 & 0xffffu, amax2 >> 16);
                 amax = max(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
                 amax = max(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-                if ((amax >> 7) != 0) {
-                    const int maxexp = (int)(amax >> 7) - 127;
-                    e = min(126, max(100, maxexp + 6)) - maxexp;
-                    cw = __uint_as_float((uint32_t)(127 + 133 - e) << 23);
-                }
+                xsc = dev::x_scale(amax);
+                cw = xsc.undo;
             }
-            // bf16 bits times 2^ee; zeros, subnormals and whatever would leave the normal range become 0
-            auto scaled = [](uint32_t b, int ee) -> uint32_t {
-                const int ex = (int)((b >> 7) & 0xffu), nx = ex + ee;
-                return (ex == 0 || nx < 1 || nx > 254) ? 0u : ((b & 0x807fu) | ((uint32_t)nx << 7));
-            };
-            auto pair = [&](uint32_t lo, uint32_t hi, int ee) { return scaled(lo & 0xffffu, ee) | (scaled(hi & 0xffffu, ee) << 16); };
             if constexpr (!BATCH && !Q8) {
                 constexpr uint32_t NW = 4 * SW;  // 8-column words of the slice: lane L < NW handles word L
                 // Every window's load first, then the processing: one L2 round trip on the launch's start-up path
@@ -678,19 +646,15 @@ __global__ void __launch_bounds__(kThreads, TESSL_GEMV_MMA_MIN_BLOCKS) q4_gemv_m
                 for (int win = 0; win < NWIN; ++win) {
                     const uint32_t xst = xstage + win * kXStageBytes;
                     const uint4 r = rw[win];
-                    uint32_t amax = max(max(r.x & 0x7fffu, (r.x >> 16) & 0x7fffu), max(r.y & 0x7fffu, (r.y >> 16) & 0x7fffu));
-                    amax = max(amax, max(max(r.z & 0x7fffu, (r.z >> 16) & 0x7fffu), max(r.w & 0x7fffu, (r.w >> 16) & 0x7fffu)));
-                    amax = __reduce_max_sync(0xffffffffu, amax);  // one instruction: this chain is the launch's start-up path
-                    e = 0, cw = 0.0f;
-                    if ((amax >> 7) != 0) {
-                        const int maxexp = (int)(amax >> 7) - 127;
-                        e = min(126, max(100, maxexp + 6)) - maxexp;
-                        cw = __uint_as_float((uint32_t)(127 + 133 - e) << 23);
-                    }
-                    cwv[win] = cw;
+                    const uint32_t amax2 = __vmaxu2(__vmaxu2(r.x & 0x7fff7fffu, r.y & 0x7fff7fffu),
+                                                    __vmaxu2(r.z & 0x7fff7fffu, r.w & 0x7fff7fffu));
+                    // one warp-reduce instruction: this chain is the launch's start-up path
+                    const dev::XScale xw = dev::x_scale(__reduce_max_sync(0xffffffffu, max(amax2 & 0xffffu, amax2 >> 16)));
+                    cwv[win] = cw = xw.undo;
                     if ((uint32_t)lane < NW) {
-                        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(xst + lane * 16), "r"(pair(r.x, r.z, e)),
-                                     "r"(pair(r.x >> 16, r.z >> 16, e - 4)), "r"(pair(r.y, r.w, e)), "r"(pair(r.y >> 16, r.w >> 16, e - 4))
+                        uint32_t f[4];
+                        dev::x_fragment(r, xw, f);
+                        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(xst + lane * 16), "r"(f[0]), "r"(f[1]), "r"(f[2]), "r"(f[3])
                                      : "memory");
                     }
                     float part = (dev::bf16_lo(r.x) + dev::bf16_hi(r.x)) + (dev::bf16_lo(r.y) + dev::bf16_hi(r.y));
@@ -708,24 +672,13 @@ __global__ void __launch_bounds__(kThreads, TESSL_GEMV_MMA_MIN_BLOCKS) q4_gemv_m
                 float part = 0.0f;
 #pragma unroll
                 for (int u = 0; u < WPG; ++u) {
-                    const uint32_t k = k0 + jj * G + t * (G / 4) + 8 * u;
-                    if constexpr (Q8) {
-                        // the word holds 4 codes; a code 0..255 read as a bf16 bit pattern is c * 2^-133 exactly (the
-                        // subnormals and the first binade form one linear scale), so (w & 0x00ff00ff) is an A register
-                        // of codes 0, 2 and ((w >> 8) & 0x00ff00ff) one of codes 1, 3: no magic constant, no offset
-                        const uint2 r = dev::ld_after_wait8(xrow + k / 2);
-                        xb[jj * WPG + u][0] = pair(r.x, r.y, e);              // x0, x2
-                        xb[jj * WPG + u][1] = pair(r.x >> 16, r.y >> 16, e);  // x1, x3
-                        part += (dev::bf16_lo(r.x) + dev::bf16_hi(r.x)) + (dev::bf16_lo(r.y) + dev::bf16_hi(r.y));
-                    } else {
-                        const uint4 r = dev::ld_after_wait16(xrow + k);
-                        xb[jj * WPG + u][0] = pair(r.x, r.z, e);                  // x0, x4
-                        xb[jj * WPG + u][1] = pair(r.x >> 16, r.z >> 16, e - 4);  // (x1, x5) / 16
-                        xb[jj * WPG + u][2] = pair(r.y, r.w, e);                  // x2, x6
-                        xb[jj * WPG + u][3] = pair(r.y >> 16, r.w >> 16, e - 4);  // (x3, x7) / 16
-                        part += (dev::bf16_lo(r.x) + dev::bf16_hi(r.x)) + (dev::bf16_lo(r.y) + dev::bf16_hi(r.y));
-                        part += (dev::bf16_lo(r.z) + dev::bf16_hi(r.z)) + (dev::bf16_lo(r.w) + dev::bf16_hi(r.w));
-                    }
+                    // the word holds 4 codes; a code 0..255 read as a bf16 bit pattern is c * 2^-133 exactly (the
+                    // subnormals and the first binade form one linear scale), so (w & 0x00ff00ff) is an A register
+                    // of codes 0, 2 and ((w >> 8) & 0x00ff00ff) one of codes 1, 3: no magic constant, no offset
+                    const uint2 r = make_uint2(xb[jj * WPG + u][0], xb[jj * WPG + u][1]);
+                    xb[jj * WPG + u][0] = dev::bf2_mul(__byte_perm(r.x, r.y, 0x5410), xsc.mul);  // x0, x2
+                    xb[jj * WPG + u][1] = dev::bf2_mul(__byte_perm(r.x, r.y, 0x7632), xsc.mul);  // x1, x3
+                    part += (dev::bf16_lo(r.x) + dev::bf16_hi(r.x)) + (dev::bf16_lo(r.y) + dev::bf16_hi(r.y));
                 }
                 part += __shfl_xor_sync(0xffffffffu, part, 1);
                 part += __shfl_xor_sync(0xffffffffu, part, 2);
@@ -758,18 +711,17 @@ __global__ void __launch_bounds__(kThreads, TESSL_GEMV_MMA_MIN_BLOCKS) q4_gemv_m
                 break;
             }
             const uint32_t st = ring + s * stage_bytes;
-            float vlo = 0.0f, vhi = 0.0f;  // M = 1: this lane's share of MMA rows g and g + 8, over all windows
-            float acc[4][4] = {};
+            float vlo = 0.0f, vhi = 0.0f;  // M = 1: the warp's share of MMA rows g and g + 8, over all windows
+            // Sums over the slice's groups, in order, of scale * dot (in units of 1 / cw) and of bias * group sum; BATCH: rows
+            // g, g + 8 x columns 2 t, 2 t + 1, else rows g, g + 8 (every lane of a quad the same: taking the groups in turn
+            // needs selects and a butterfly, which cost more than the products they save).
+            float as[4], ab[4];
 #pragma unroll
             for (int win = 0; win < NWIN; ++win) {
             if constexpr (NWIN > 1) load_x(win), cw = cwv[win];
             const uint32_t row_lo = st + row_base + win * (KW >> 1), row_hi = row_lo + row_bytes;
             const uint32_t sb_lo = st + sb_base + win * ((KW >> p.group_shift) * 4);
             const uint32_t sb_hi = sb_lo + sb_row_bytes;
-            float dlo[NGS], dhi[NGS];        // M = 1: dot of MMA rows g and g + 8 per group
-            // BATCH: rows g, g + 8 x columns 2 t, 2 t + 1, one accumulator per group class jj % 4 so that
-            // the sum is formed in the same order as in the M = 1 path (where lane t of a quad takes
-            // the groups t, t + 4, ... and the quad is then added up by a butterfly)
             // All words of the slice first (the rows were copied long ago: these loads do not wait),
             // then the MMAs interleaved over the groups: consecutive MMAs belong to different
             // accumulator chains, so none waits for its predecessor. Within a chain the order is
@@ -815,50 +767,47 @@ __global__ void __launch_bounds__(kThreads, TESSL_GEMV_MMA_MIN_BLOCKS) q4_gemv_m
                 }
             }
 #pragma unroll
+            for (int c = 0; c < 4; ++c) as[c] = ab[c] = 0.0f;
+            uint32_t pl[NGS], ph2[NGS];  // the rows' scale/bias pairs: aligned vectors of up to four
+            if constexpr (NGS % 4 == 0) {
+#pragma unroll
+                for (int q = 0; q < NGS; q += 4) {
+                    const uint4 a = q4k::lds128(sb_lo + 4 * q), b = q4k::lds128(sb_hi + 4 * q);
+                    pl[q] = a.x, pl[q + 1] = a.y, pl[q + 2] = a.z, pl[q + 3] = a.w;
+                    ph2[q] = b.x, ph2[q + 1] = b.y, ph2[q + 2] = b.z, ph2[q + 3] = b.w;
+                }
+            } else if constexpr (NGS == 2) {
+                const uint2 a = lds64(sb_lo), b = lds64(sb_hi);
+                pl[0] = a.x, pl[1] = a.y, ph2[0] = b.x, ph2[1] = b.y;
+            } else {
+                pl[0] = lds32(sb_lo), ph2[0] = lds32(sb_hi);
+            }
+#pragma unroll
             for (int jj = 0; jj < NGS; ++jj) {
+                const float sl = dev::bf16_lo(pl[jj]), bl = dev::bf16_hi(pl[jj]), sh = dev::bf16_lo(ph2[jj]), bh = dev::bf16_hi(ph2[jj]);
+                as[0] = fmaf(sl, d[jj][0], as[0]), as[2] = fmaf(sh, d[jj][2], as[2]);
                 if constexpr (BATCH) {
-                    const uint32_t pl = lds32(sb_lo + jj * 4), ph2 = lds32(sb_hi + jj * 4);
-                    const float sl = dev::bf16_lo(pl), bl = dev::bf16_hi(pl), sh = dev::bf16_lo(ph2), bh = dev::bf16_hi(ph2);
-                    const int cls = jj & 3;  // a constant once the loop is unrolled
-                    acc[0][cls] = fmaf(sl, d[jj][0] * cw0, fmaf(bl, xs0[jj], acc[0][cls]));
-                    acc[1][cls] = fmaf(sl, d[jj][1] * cw1, fmaf(bl, xs1[jj], acc[1][cls]));
-                    acc[2][cls] = fmaf(sh, d[jj][2] * cw0, fmaf(bh, xs0[jj], acc[2][cls]));
-                    acc[3][cls] = fmaf(sh, d[jj][3] * cw1, fmaf(bh, xs1[jj], acc[3][cls]));
+                    as[1] = fmaf(sl, d[jj][1], as[1]), as[3] = fmaf(sh, d[jj][3], as[3]);
+                    ab[0] = fmaf(bl, xs0[jj], ab[0]), ab[1] = fmaf(bl, xs1[jj], ab[1]);
+                    ab[2] = fmaf(bh, xs0[jj], ab[2]), ab[3] = fmaf(bh, xs1[jj], ab[3]);
                 } else {
-                    dlo[jj] = d[jj][0], dhi[jj] = d[jj][2];  // every column holds the same vector: d[1] == d[0]
+                    ab[0] = fmaf(bl, xs[jj], ab[0]), ab[2] = fmaf(bh, xs[jj], ab[2]);  // every column holds the same vector
                 }
             }
             if constexpr (!BATCH) {
-                // The four lanes of a quad hold the same dots: lane t folds the affine of groups t, t + 4, ...
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) {
-                    float dl = 0.0f, dh = 0.0f, xg = 0.0f;
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        if (4 * q + i < NGS && t == (uint32_t)i) dl = dlo[4 * q + i], dh = dhi[4 * q + i], xg = xs[4 * q + i];
-                    const uint32_t jj = 4 * q + t;
-                    if (jj < (uint32_t)NGS) {
-                        const uint32_t pl = lds32(sb_lo + jj * 4), ph2 = lds32(sb_hi + jj * 4);
-                        vlo = fmaf(dev::bf16_lo(pl), dl * cw, fmaf(dev::bf16_hi(pl), xg, vlo));
-                        vhi = fmaf(dev::bf16_lo(ph2), dh * cw, fmaf(dev::bf16_hi(ph2), xg, vhi));
-                    }
-                }
+                const float lo = fmaf(cw, as[0], ab[0]), hi = fmaf(cw, as[2], ab[2]);
+                vlo = win == 0 ? lo : vlo + lo, vhi = win == 0 ? hi : vhi + hi;
             }
             }  // windows
             const uint32_t part = st + off_part;
             if constexpr (BATCH) {
-                float o[4];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) o[c] = (acc[c][0] + acc[c][1]) + (acc[c][2] + acc[c][3]);
-                asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(part + ((warp * 16 + g) * 8 + 2 * t) * 4), "f"(o[0]),
-                             "f"(o[1])
+                asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(part + ((warp * 16 + g) * 8 + 2 * t) * 4),
+                             "f"(fmaf(cw0, as[0], ab[0])), "f"(fmaf(cw1, as[1], ab[1]))
                              : "memory");
                 asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(part + ((warp * 16 + g + 8) * 8 + 2 * t) * 4),
-                             "f"(o[2]), "f"(o[3])
+                             "f"(fmaf(cw0, as[2], ab[2])), "f"(fmaf(cw1, as[3], ab[3]))
                              : "memory");
             } else {
-                vlo += __shfl_xor_sync(0xffffffffu, vlo, 1), vhi += __shfl_xor_sync(0xffffffffu, vhi, 1);
-                vlo += __shfl_xor_sync(0xffffffffu, vlo, 2), vhi += __shfl_xor_sync(0xffffffffu, vhi, 2);
                 if (t == 0) {
                     asm volatile("st.shared.f32 [%0], %1;" ::"r"(part + (warp * 16 + g) * 4), "f"(vlo) : "memory");
                     asm volatile("st.shared.f32 [%0], %1;" ::"r"(part + (warp * 16 + g + 8) * 4), "f"(vhi) : "memory");

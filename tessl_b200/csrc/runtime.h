@@ -15,6 +15,7 @@
 #include <map>
 #include <string>
 #include <thread>
+#include <utility>
 
 #include "../../include/tessl_b200.h"
 
@@ -56,6 +57,8 @@ struct TesslRuntime {
     // Dynamic shared memory already opted in, per kernel. The attribute belongs to the
     // device's context, so it is remembered per runtime (one device each), not per process.
     std::map<const void *, size_t> smem_opted;
+    // Clusters of a given size that the device holds at once, per kernel (asked once).
+    std::map<std::pair<const void *, uint32_t>, int> max_clusters;
     // Prefill GEMM tile choice: what a tuning run or a test asked for (0 / -1 = the library
     // decides) and what the last call ran (0 = no tile kernel ran, e.g. the small-batch route).
     int prefill_force_bn = 0;
