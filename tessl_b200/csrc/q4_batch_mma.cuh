@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(kThreads, 1) q4_batch_mma_kernel(const __grid_
                 }
                 part += __shfl_xor_sync(0xffffffffu, part, 1);
                 part += __shfl_xor_sync(0xffffffffu, part, 2);
-                xs[jj] = part;  // the same in the four lanes of a quad
+                xs[jj] = dev::scaled_sum(part, xsc);  // the same in the four lanes of a quad
             }
         }
         // this lane's outputs are batch columns 2 t and 2 t + 1; their group sums live in quads 2 t and 2 t + 1
@@ -394,9 +394,9 @@ __global__ void __launch_bounds__(kThreads, 1) q4_batch_mma_kernel(const __grid_
                 break;
             }
             const uint32_t st = ring + s * stage_bytes;
-            // rows rl, rl + 8 x columns 2 t, 2 t + 1: sums over the groups, in order, of scale * dot (in units of 1 / cw)
-            // and of bias * group sum
-            float as[4] = {}, ab[4] = {};
+            // rows rl, rl + 8 x columns 2 t, 2 t + 1: the groups' scale * dot + bias * group sum in units of cw, one
+            // accumulator per group class jj % 4 (the order of q4_gemv_mma.cuh)
+            float acc[4][4] = {};
 #pragma unroll
             for (int b0 = 0; b0 < NGS; b0 += 4) {  // four groups at a time: their MMA chains are interleaved
                 uint32_t wl[4 * WPG], wh[4 * WPG], sl[4], sh[4];
@@ -451,17 +451,19 @@ __global__ void __launch_bounds__(kThreads, 1) q4_batch_mma_kernel(const __grid_
                     if (b0 + i >= NGS) continue;
                     if (EVEN || b0 + i < NGS - 1 || whole) {
                         const float s0 = dev::bf16_lo(sl[i]), z0 = dev::bf16_hi(sl[i]), s1 = dev::bf16_lo(sh[i]), z1 = dev::bf16_hi(sh[i]);
-                        as[0] = fmaf(s0, d[i][0], as[0]), as[1] = fmaf(s0, d[i][1], as[1]);
-                        as[2] = fmaf(s1, d[i][2], as[2]), as[3] = fmaf(s1, d[i][3], as[3]);
-                        ab[0] = fmaf(z0, xs0[b0 + i], ab[0]), ab[1] = fmaf(z0, xs1[b0 + i], ab[1]);
-                        ab[2] = fmaf(z1, xs0[b0 + i], ab[2]), ab[3] = fmaf(z1, xs1[b0 + i], ab[3]);
+                        acc[0][i] = fmaf(s0, d[i][0], fmaf(z0, xs0[b0 + i], acc[0][i]));
+                        acc[1][i] = fmaf(s0, d[i][1], fmaf(z0, xs1[b0 + i], acc[1][i]));
+                        acc[2][i] = fmaf(s1, d[i][2], fmaf(z1, xs0[b0 + i], acc[2][i]));
+                        acc[3][i] = fmaf(s1, d[i][3], fmaf(z1, xs1[b0 + i], acc[3][i]));
                     }
                 }
             }
-            asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(st + part_off), "f"(fmaf(cw0, as[0], ab[0])), "f"(fmaf(cw1, as[1], ab[1]))
+            float o[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) o[c] = ((acc[c][0] + acc[c][1]) + (acc[c][2] + acc[c][3])) * (c & 1 ? cw1 : cw0);
+            asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(st + part_off), "f"(o[0]), "f"(o[1])
                          : "memory");
-            asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(st + part_off + 256), "f"(fmaf(cw0, as[2], ab[2])),
-                         "f"(fmaf(cw1, as[3], ab[3]))
+            asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(st + part_off + 256), "f"(o[2]), "f"(o[3])
                          : "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(done(s));  // release: the partial sums are visible to the reducer

@@ -52,17 +52,20 @@ __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w 
 /// Power-of-two scaling of a slice of bf16 activations that meets nibbles held as bf16 subnormals (q * 2^-133): `mul` =
 /// (2^e, 2^e) and `mul16` = (2^(e-4), 2^(e-4)) as bf16 pairs, `undo` = 2^(133-e). e brings the slice's largest magnitude
 /// to about 2^100, so that every product is a normal f32, within what a bf16 factor (e <= 127) and an f32 undo (e >= 6)
-/// can hold. `amax`: the largest magnitude's bits; a slice of zeros and subnormals counts as zero.
+/// can hold. The affine fold of the slice then runs in units of `undo` (`scaled_sum`: a group sum in those units): the
+/// same roundings as on the plain values, without a multiplication per dot product. `amax`: the largest magnitude's bits.
 struct XScale {
     uint32_t mul, mul16;
-    float undo;
+    float undo, sum1;
 };
 __device__ __forceinline__ XScale x_scale(uint32_t amax)
 {
-    if ((amax >> 7) == 0) return XScale{0u, 0u, 0.0f};
     const int e = min(127, max(6, 100 + 127 - (int)(amax >> 7)));
-    return XScale{(uint32_t)(e + 127) * 0x00800080u, (uint32_t)(e + 123) * 0x00800080u, __uint_as_float((uint32_t)(127 + 133 - e) << 23)};
+    return XScale{(uint32_t)(e + 127) * 0x00800080u, (uint32_t)(e + 123) * 0x00800080u, __uint_as_float((uint32_t)(127 + 133 - e) << 23),
+                  __uint_as_float((uint32_t)(e + 57) << 23)};
 }
+/// sum * 2^(e - 133), in two factors that are normal for every e.
+__device__ __forceinline__ float scaled_sum(float sum, const XScale &s) { return sum * s.sum1 * 0x1p-63f; }
 __device__ __forceinline__ uint32_t bf2_mul(uint32_t a, uint32_t b)
 {
     uint32_t r;

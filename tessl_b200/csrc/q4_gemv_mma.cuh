@@ -204,7 +204,8 @@ __global__ void __launch_bounds__(kThreads, TESSL_GEMV_MMA_MIN_BLOCKS) q4_gemv_m
     static_assert(ROWS % (2 * NB) == 0 && ROWS <= 16, "whole row pairs per bank");
     constexpr int NGS = SW / WPG;     // groups per slice
     constexpr int RPB = ROWS / NB;    // rows per bank and stage
-    static_assert(SW % WPG == 0 && (NGS == 1 || NGS == 2 || NGS % 4 == 0), "a warp's slice holds whole groups");
+    constexpr int NQ = (NGS + 3) / 4;  // affine groups per lane when M = 1
+    static_assert(SW % WPG == 0 && NGS >= 1, "a warp's slice holds whole groups");
     static_assert(!BATCH || Q8, "Q4 batches run on q4_batch_mma.cuh");
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ int abort_flag;
@@ -661,7 +662,8 @@ __global__ void __launch_bounds__(kThreads, TESSL_GEMV_MMA_MIN_BLOCKS) q4_gemv_m
                     part += (dev::bf16_lo(r.z) + dev::bf16_hi(r.z)) + (dev::bf16_lo(r.w) + dev::bf16_hi(r.w));
 #pragma unroll
                     for (int o = 1; o < 4 * WPG && o < 32; o <<= 1) part += __shfl_xor_sync(0xffffffffu, part, o);  // a group: 4 WPG lanes
-                    const float gsum = __shfl_sync(0xffffffffu, part, (lane * 4 * WPG) & 31);
+                    float gsum = __shfl_sync(0xffffffffu, part, (lane * 4 * WPG) & 31);
+                    if constexpr (NWIN == 1) gsum = dev::scaled_sum(gsum, xw);  // one window: the fold runs in units of cw
                     if (lane < NGS) asm volatile("st.shared.f32 [%0], %1;" ::"r"(xst + 512 + lane * 4), "f"(gsum) : "memory");
                 }
                 __syncwarp();
@@ -682,7 +684,7 @@ __global__ void __launch_bounds__(kThreads, TESSL_GEMV_MMA_MIN_BLOCKS) q4_gemv_m
                 }
                 part += __shfl_xor_sync(0xffffffffu, part, 1);
                 part += __shfl_xor_sync(0xffffffffu, part, 2);
-                xs[jj] = part;  // the same in the four lanes of a quad
+                xs[jj] = dev::scaled_sum(part, xsc);  // the same in the four lanes of a quad
             }
         }
         // BATCH: this lane's outputs are batch columns 2 t and 2 t + 1; their group sums live in quads 2 t and 2 t + 1.
@@ -712,10 +714,10 @@ __global__ void __launch_bounds__(kThreads, TESSL_GEMV_MMA_MIN_BLOCKS) q4_gemv_m
             }
             const uint32_t st = ring + s * stage_bytes;
             float vlo = 0.0f, vhi = 0.0f;  // M = 1: the warp's share of MMA rows g and g + 8, over all windows
-            // Sums over the slice's groups, in order, of scale * dot (in units of 1 / cw) and of bias * group sum; BATCH: rows
-            // g, g + 8 x columns 2 t, 2 t + 1, else rows g, g + 8 (every lane of a quad the same: taking the groups in turn
-            // needs selects and a butterfly, which cost more than the products they save).
-            float as[4], ab[4];
+            // BATCH: rows g, g + 8 x columns 2 t, 2 t + 1, one accumulator per group class jj % 4 so that the sum is formed in
+            // the same order as in the M = 1 path (where lane t of a quad takes the groups t, t + 4, ... and the quad is
+            // then added up by a butterfly; every lane taking all groups in turn is a longer chain: gate/up 11.2 -> 12.0 us)
+            float acc[4][4] = {};
 #pragma unroll
             for (int win = 0; win < NWIN; ++win) {
             if constexpr (NWIN > 1) load_x(win), cw = cwv[win];
@@ -766,48 +768,51 @@ __global__ void __launch_bounds__(kThreads, TESSL_GEMV_MMA_MIN_BLOCKS) q4_gemv_m
                     }
                 }
             }
+            if constexpr (BATCH) {
 #pragma unroll
-            for (int c = 0; c < 4; ++c) as[c] = ab[c] = 0.0f;
-            uint32_t pl[NGS], ph2[NGS];  // the rows' scale/bias pairs: aligned vectors of up to four
-            if constexpr (NGS % 4 == 0) {
-#pragma unroll
-                for (int q = 0; q < NGS; q += 4) {
-                    const uint4 a = q4k::lds128(sb_lo + 4 * q), b = q4k::lds128(sb_hi + 4 * q);
-                    pl[q] = a.x, pl[q + 1] = a.y, pl[q + 2] = a.z, pl[q + 3] = a.w;
-                    ph2[q] = b.x, ph2[q + 1] = b.y, ph2[q + 2] = b.z, ph2[q + 3] = b.w;
+                for (int jj = 0; jj < NGS; ++jj) {
+                    const uint32_t pl = lds32(sb_lo + jj * 4), ph2 = lds32(sb_hi + jj * 4);
+                    const float sl = dev::bf16_lo(pl), bl = dev::bf16_hi(pl), sh = dev::bf16_lo(ph2), bh = dev::bf16_hi(ph2);
+                    const int cls = jj & 3;  // a constant once the loop is unrolled
+                    acc[0][cls] = fmaf(sl, d[jj][0], fmaf(bl, xs0[jj], acc[0][cls]));
+                    acc[1][cls] = fmaf(sl, d[jj][1], fmaf(bl, xs1[jj], acc[1][cls]));
+                    acc[2][cls] = fmaf(sh, d[jj][2], fmaf(bh, xs0[jj], acc[2][cls]));
+                    acc[3][cls] = fmaf(sh, d[jj][3], fmaf(bh, xs1[jj], acc[3][cls]));
                 }
-            } else if constexpr (NGS == 2) {
-                const uint2 a = lds64(sb_lo), b = lds64(sb_hi);
-                pl[0] = a.x, pl[1] = a.y, ph2[0] = b.x, ph2[1] = b.y;
             } else {
-                pl[0] = lds32(sb_lo), ph2[0] = lds32(sb_hi);
-            }
+                // The four lanes of a quad hold the same dots (every column holds the same vector: d[1] == d[0]): lane t folds
+                // the affine of groups t, t + 4, ...
 #pragma unroll
-            for (int jj = 0; jj < NGS; ++jj) {
-                const float sl = dev::bf16_lo(pl[jj]), bl = dev::bf16_hi(pl[jj]), sh = dev::bf16_lo(ph2[jj]), bh = dev::bf16_hi(ph2[jj]);
-                as[0] = fmaf(sl, d[jj][0], as[0]), as[2] = fmaf(sh, d[jj][2], as[2]);
-                if constexpr (BATCH) {
-                    as[1] = fmaf(sl, d[jj][1], as[1]), as[3] = fmaf(sh, d[jj][3], as[3]);
-                    ab[0] = fmaf(bl, xs0[jj], ab[0]), ab[1] = fmaf(bl, xs1[jj], ab[1]);
-                    ab[2] = fmaf(bh, xs0[jj], ab[2]), ab[3] = fmaf(bh, xs1[jj], ab[3]);
-                } else {
-                    ab[0] = fmaf(bl, xs[jj], ab[0]), ab[2] = fmaf(bh, xs[jj], ab[2]);  // every column holds the same vector
+                for (int q = 0; q < NQ; ++q) {
+                    float dl = 0.0f, dh = 0.0f, xg = 0.0f;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (4 * q + i < NGS && t == (uint32_t)i) dl = d[4 * q + i][0], dh = d[4 * q + i][2], xg = xs[4 * q + i];
+                    const uint32_t jj = 4 * q + t;
+                    if (jj < (uint32_t)NGS) {
+                        const uint32_t pl = lds32(sb_lo + jj * 4), ph2 = lds32(sb_hi + jj * 4);
+                        if constexpr (NWIN > 1) dl *= cw, dh *= cw;  // each window has its own unit
+                        vlo = fmaf(dev::bf16_lo(pl), dl, fmaf(dev::bf16_hi(pl), xg, vlo));
+                        vhi = fmaf(dev::bf16_lo(ph2), dh, fmaf(dev::bf16_hi(ph2), xg, vhi));
+                    }
                 }
-            }
-            if constexpr (!BATCH) {
-                const float lo = fmaf(cw, as[0], ab[0]), hi = fmaf(cw, as[2], ab[2]);
-                vlo = win == 0 ? lo : vlo + lo, vhi = win == 0 ? hi : vhi + hi;
             }
             }  // windows
             const uint32_t part = st + off_part;
             if constexpr (BATCH) {
-                asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(part + ((warp * 16 + g) * 8 + 2 * t) * 4),
-                             "f"(fmaf(cw0, as[0], ab[0])), "f"(fmaf(cw1, as[1], ab[1]))
+                float o[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) o[c] = ((acc[c][0] + acc[c][1]) + (acc[c][2] + acc[c][3])) * (c & 1 ? cw1 : cw0);
+                asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(part + ((warp * 16 + g) * 8 + 2 * t) * 4), "f"(o[0]),
+                             "f"(o[1])
                              : "memory");
                 asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(part + ((warp * 16 + g + 8) * 8 + 2 * t) * 4),
-                             "f"(fmaf(cw0, as[2], ab[2])), "f"(fmaf(cw1, as[3], ab[3]))
+                             "f"(o[2]), "f"(o[3])
                              : "memory");
             } else {
+                vlo += __shfl_xor_sync(0xffffffffu, vlo, 1), vhi += __shfl_xor_sync(0xffffffffu, vhi, 1);
+                vlo += __shfl_xor_sync(0xffffffffu, vlo, 2), vhi += __shfl_xor_sync(0xffffffffu, vhi, 2);
+                if constexpr (NWIN == 1) vlo *= cw, vhi *= cw;
                 if (t == 0) {
                     asm volatile("st.shared.f32 [%0], %1;" ::"r"(part + (warp * 16 + g) * 4), "f"(vlo) : "memory");
                     asm volatile("st.shared.f32 [%0], %1;" ::"r"(part + (warp * 16 + g + 8) * 4), "f"(vhi) : "memory");
