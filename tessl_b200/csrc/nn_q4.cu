@@ -28,16 +28,54 @@ using q4k::EPI_STORE;
 using Q4Seg = q4k::Seg;
 using Q4GemvParams = q4k::Params;
 
-__global__ void swiglu_kernel(const float *gate, const float *up, void *out, uint32_t n, int out_bf16, int gelu)
+/// silu(gate) * up (or GELU), four neighbouring elements per thread where the buffers allow 16-byte accesses (VEC = 4).
+/// Bound by its 10 (bf16) or 12 bytes per element; with one element per thread a prompt's 509 x 6144 was bound by its
+/// load instructions.
+template <int VEC>
+__global__ void __launch_bounds__(256) swiglu_kernel(const float *gate, const float *up, void *out, uint32_t n, int out_bf16, int gelu)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * VEC;
     if (i >= n) return;
-    const float v = (gelu ? dev::gelu_pytorch_tanh(gate[i]) : dev::silu(gate[i])) * up[i];
-    if (out_bf16) {
-        static_cast<uint16_t *>(out)[i] = dev::f32_to_bf16_store(v);
+    float g[VEC], u[VEC];
+    if constexpr (VEC == 4) {
+        const uint4 a = dev::ld_after_wait16(gate + i), b = dev::ld_after_wait16(up + i);
+        g[0] = __uint_as_float(a.x), g[1] = __uint_as_float(a.y), g[2] = __uint_as_float(a.z), g[3] = __uint_as_float(a.w);
+        u[0] = __uint_as_float(b.x), u[1] = __uint_as_float(b.y), u[2] = __uint_as_float(b.z), u[3] = __uint_as_float(b.w);
     } else {
-        static_cast<float *>(out)[i] = v;
+        g[0] = *(volatile const float *)(gate + i), u[0] = *(volatile const float *)(up + i);
     }
+    float v[VEC];
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) v[k] = (gelu ? dev::gelu_pytorch_tanh(g[k]) : dev::silu(g[k])) * u[k];
+    if (out_bf16) {
+        uint16_t h[VEC];
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) h[k] = dev::f32_to_bf16_store(v[k]);
+        uint16_t *o = static_cast<uint16_t *>(out) + i;
+        if constexpr (VEC == 4) {
+            *reinterpret_cast<uint2 *>(o) = make_uint2((uint32_t)h[0] | ((uint32_t)h[1] << 16), (uint32_t)h[2] | ((uint32_t)h[3] << 16));
+        } else {
+            o[0] = h[0];
+        }
+    } else {
+        float *o = static_cast<float *>(out) + i;
+        if constexpr (VEC == 4) {
+            *reinterpret_cast<float4 *>(o) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+            o[0] = v[0];
+        }
+    }
+}
+
+Result launch_swiglu(TesslRuntime *rt, const char *what, const float *gate, const float *up, void *out, uint32_t n, int out_bf16, int gelu)
+{
+    const bool vec = n % 4 == 0 && (((uintptr_t)gate | (uintptr_t)up) & 15u) == 0 && ((uintptr_t)out & (out_bf16 ? 7u : 15u)) == 0;
+    const uint32_t work = vec ? n / 4 : n;
+    const dim3 grid(work / 256 + (work % 256 != 0));
+    if (vec) return launch_pdl(rt, what, swiglu_kernel<4>, grid, dim3(256), 0, gate, up, out, n, out_bf16, gelu);
+    return launch_pdl(rt, what, swiglu_kernel<1>, grid, dim3(256), 0, gate, up, out, n, out_bf16, gelu);
 }
 
 __global__ void q4_unpack_kernel(const uint8_t *packed, uint8_t *out, uint64_t n_bytes)
@@ -109,11 +147,13 @@ __global__ void q4_dequant_kernel(const uint8_t *packed, const uint32_t *sb, flo
 __global__ void embed_lookup_q4_mlx_kernel(const uint8_t *packed, const uint32_t *sb, const uint32_t *token_ids, float *out,
                                            uint32_t hidden, uint32_t group_shift, uint32_t vocab, uint64_t total32)
 {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total32) return;
     const uint32_t per_row = hidden / 32;
     const uint32_t m = (uint32_t)(i / per_row), c = (uint32_t)(i % per_row);
-    const uint32_t tid = token_ids[m];
+    const uint32_t tid = *(volatile const uint32_t *)(token_ids + m);
     float4 *o = reinterpret_cast<float4 *>(out + (size_t)m * hidden + (size_t)c * 32);
     if (tid >= vocab) {
 #pragma unroll
@@ -638,10 +678,7 @@ Result launch_q4_gemv(TesslRuntime *rt, Q4GemvParams p, int m, int nb)
         TESSL_TRY(launch_mma_long(rt, q));
         q.seg[0].packed0 = p.seg[0].packed1, q.seg[0].sb0 = p.seg[0].sb1, q.seg[0].out = u;
         TESSL_TRY(launch_mma_long(rt, q));
-        swiglu_kernel<<<(rows + 255) / 256, 256, 0, rt->stream>>>(g, u, p.seg[0].out, rows, p.out_bf16,
-                                                                  p.epi == EPI_GATE_UP_GELU ? 1 : 0);
-        rt->dispatch_count += 1;
-        TESSL_TRY(cuda_check(rt, cudaGetLastError(), "gate/up activation launch"));
+        TESSL_TRY(launch_swiglu(rt, "gate/up activation launch", g, u, p.seg[0].out, rows, p.out_bf16, p.epi == EPI_GATE_UP_GELU ? 1 : 0));
         if (p.peer) return nn::peer_gather(rt, *static_cast<const TesslPeerGather *>(p.peer));
         return ok();
     }
@@ -1062,11 +1099,8 @@ Result swiglu(TesslRuntime *rt, const TesslBuf &gate, const TesslBuf &up, const 
     TESSL_TRY(require(up, n, 4, "swiglu up"));
     TESSL_TRY(require(out, n, out_as_bf16 ? 2 : 4, "swiglu out"));
     if (n == 0) return ok();
-    swiglu_kernel<<<(n + 255) / 256, 256, 0, rt->stream>>>(static_cast<const float *>(gate.ptr),
-                                                          static_cast<const float *>(up.ptr), out.ptr, n,
-                                                          out_as_bf16 ? 1 : 0, 0);
-    rt->dispatch_count += 1;
-    return cuda_check(rt, cudaGetLastError(), "swiglu launch");
+    return launch_swiglu(rt, "swiglu launch", static_cast<const float *>(gate.ptr), static_cast<const float *>(up.ptr), out.ptr, n,
+                         out_as_bf16 ? 1 : 0, 0);
 }
 
 /// A validated prefill call with few rows, run as batches of up to 8 rows on the tensor-core GEMV kernel:
@@ -1148,12 +1182,10 @@ Result embed_lookup_q4_mlx(TesslRuntime *rt, const TesslQ4MlxBank &bank, const T
     TESSL_TRY(require_aligned16(out, std::string(what) + " out"));
     if (((uintptr_t)token_ids.ptr & 3u) != 0) return fmt("%s token_ids: device pointer must be 4-byte aligned", what);
     const uint64_t total32 = total / 32;  // hidden is a multiple of the group size, itself a multiple of 32
-    embed_lookup_q4_mlx_kernel<<<(unsigned)((total32 + 127) / 128), 128, 0, rt->stream>>>(
-        static_cast<const uint8_t *>(bank.packed.ptr), static_cast<const uint32_t *>(bank.scales_biases.ptr),
-        static_cast<const uint32_t *>(token_ids.ptr), static_cast<float *>(out.ptr), hidden, log2_u32(group_size), vocab,
-        total32);
-    rt->dispatch_count += 1;
-    return cuda_check(rt, cudaGetLastError(), "embed_lookup_q4_mlx launch");
+    return launch_pdl(rt, "embed_lookup_q4_mlx launch", embed_lookup_q4_mlx_kernel, dim3((unsigned)((total32 + 127) / 128)), dim3(128), 0,
+                      static_cast<const uint8_t *>(bank.packed.ptr), static_cast<const uint32_t *>(bank.scales_biases.ptr),
+                      static_cast<const uint32_t *>(token_ids.ptr), static_cast<float *>(out.ptr), hidden, log2_u32(group_size), vocab,
+                      total32);
 }
 
 uint64_t q4_mlx_staged_bytes(uint32_t rows, uint32_t cols, uint32_t group_size)

@@ -68,6 +68,10 @@ using nn::OUT_BF16;
 __global__ void __launch_bounds__(256) x_prepare_kernel(const uint16_t *x, __half *a_aug, float *row_scale, uint32_t K,
                                                         uint32_t K64, uint32_t K_aug, uint32_t gshift)
 {
+    // Wait first, then let the GEMM start: its blocks set themselves up and stream weights while these rows are converted,
+    // and everything in front of this kernel is complete when they do (2 - 4 us per call).
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t m = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint16_t *xrow = x + (size_t)m * K;
     __half *arow = a_aug + (size_t)m * K_aug;
@@ -77,7 +81,7 @@ __global__ void __launch_bounds__(256) x_prepare_kernel(const uint16_t *x, __hal
     // pass 1: largest magnitude (bf16 bit patterns order like integers); Inf/NaN disable the rescale
     uint32_t amax = 0;
     for (uint32_t ch = tid; ch < K / 8; ch += 256) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(xrow) + ch);
+        const uint4 v = dev::ld_after_wait16(reinterpret_cast<const uint4 *>(xrow) + ch);
         const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) amax = max(amax, max(w[j] & 0x7fffu, (w[j] >> 16) & 0x7fffu));
@@ -109,7 +113,7 @@ __global__ void __launch_bounds__(256) x_prepare_kernel(const uint16_t *x, __hal
         const uint32_t ch = base + tid;
         float f[8];
         if (ch * 8 < K) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(xrow) + ch);
+            const uint4 v = dev::ld_after_wait16(reinterpret_cast<const uint4 *>(xrow) + ch);
             const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -415,9 +419,7 @@ Result launch_gemm_pair(TesslRuntime *rt, const CUtensorMap &ma, const CUtensorM
     TESSL_TRY(smem_opt_in(rt, reinterpret_cast<const void *>(kernel), C::SMEM, "gemm_q4_mlx_tensorops: shared memory opt-in"));
     const uint32_t tiles = p.tiles_m * p.tiles_n;
     const uint32_t clusters = std::min<uint32_t>(tiles, (uint32_t)rt->sm_count / 2);
-    kernel<<<2 * clusters, C::THREADS, C::SMEM, rt->stream>>>(ma, mw, p);
-    rt->dispatch_count += 1;
-    return cuda_check(rt, cudaGetLastError(), "gemm_q4_mlx_tensorops launch");
+    return launch_pdl(rt, "gemm_q4_mlx_tensorops launch", kernel, dim3(2 * clusters), dim3(C::THREADS), C::SMEM, ma, mw, p);
 }
 
 /// Shapes and scratch layout of one prefill GEMM call.
@@ -500,10 +502,8 @@ Result prefill_launch(TesslRuntime *rt, const TesslQ4MlxBank &bank, const TesslB
 {
     __half *a_aug = static_cast<__half *>(scratch);
     float *row_scale = reinterpret_cast<float *>(static_cast<char *>(scratch) + pl.a_bytes);
-    x_prepare_kernel<<<m, 256, 0, rt->stream>>>(static_cast<const uint16_t *>(x_bf16.ptr), a_aug, row_scale, pl.k, pl.k64,
-                                                pl.k_aug, pl.gshift);
-    rt->dispatch_count += 1;
-    TESSL_TRY(cuda_check(rt, cudaGetLastError(), "gemm_q4_mlx_tensorops pre-pass launch"));
+    TESSL_TRY(launch_pdl(rt, "gemm_q4_mlx_tensorops pre-pass launch", x_prepare_kernel, dim3(m), dim3(256), 0,
+                         static_cast<const uint16_t *>(x_bf16.ptr), a_aug, row_scale, pl.k, pl.k64, pl.k_aug, pl.gshift));
 
     const bool pair = rt->sm_count >= 2 && rt->prefill_force_pair != 0;
     const uint32_t tiles_m = pair ? (m + 2 * BM - 1) / (2 * BM) : (m + BM - 1) / BM;

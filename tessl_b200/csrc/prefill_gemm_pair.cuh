@@ -61,6 +61,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<BN>::THREADS
                                 const GemmParams p)
 {
     using C = PairCfg<BN>;
+    asm volatile("griddepcontrol.launch_dependents;");
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
@@ -118,6 +119,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<BN>::THREADS
     if (warp == 0) {
         // ------------------------------------------------ TMA producer: X tiles ---
         if (lane == 0) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");  // the pre-pass writes the activations
             RingPos<C::SA> ring;
             bool ok_ = true;
             for (uint32_t t = cluster_id; t < ntiles && ok_; t += nclusters) {
@@ -215,6 +217,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<BN>::THREADS
     } else if (warp < C::FIRST_DW) {
         // ------------------------------------------------ epilogue ---
         const uint32_t quarter = (uint32_t)warp & 3u;  // the TMEM lanes this warp may read
+        asm volatile("griddepcontrol.wait;" ::: "memory");  // row scales come from the pre-pass; y belongs to the stream's order
         uint32_t it = 0;
         for (uint32_t t = cluster_id; t < ntiles; t += nclusters, ++it) {
             const uint32_t buf = it & 1u;
@@ -225,7 +228,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<BN>::THREADS
             tcgen05_fence_after();
             const uint32_t m_base = ((t % p.tiles_m) * 2 + rank) * BM + quarter * 32;
             const uint32_t n0 = (t / p.tiles_m) * BN;
-            const float rs = m_base + lane < p.M ? p.row_scale[m_base + lane] : 0.0f;
+            const float rs = m_base + lane < p.M ? *(volatile const float *)(p.row_scale + m_base + lane) : 0.0f;
             const uint32_t stage = base + C::OFF_STAGE + quarter * 4096;
 #pragma unroll 1
             for (uint32_t c = 0; c < BN / 32; ++c) {

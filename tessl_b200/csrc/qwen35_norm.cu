@@ -93,20 +93,6 @@ __global__ void qwen35_residual_add_kernel(const float *y, float *resid, uint64_
     if (i < n) resid[i] = resid[i] + y[i];
 }
 
-template <typename K, typename... A>
-Result launch_pdl(TesslRuntime *rt, K kernel, dim3 grid, dim3 block, const char *what, A... args)
-{
-    cudaLaunchConfig_t lc{};
-    lc.gridDim = grid, lc.blockDim = block, lc.dynamicSmemBytes = 0, lc.stream = rt->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    lc.attrs = attr, lc.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&lc, kernel, args...);
-    rt->dispatch_count += 1;
-    return cuda_check(rt, e, what);
-}
-
 /// `nn::validate_rms_scalars` (src/nn.rs:190-202 of the reference project).
 Result validate_rms_scalars(uint32_t dim, float eps, const char *what)
 {
@@ -150,9 +136,9 @@ Result qwen35_rms_norm(TesslRuntime *rt, const TesslBuf &x, const TesslBuf &w, c
     float *xp = static_cast<float *>(x.ptr);
     const float *wp = static_cast<const float *>(w.ptr);
     if (out_as_bf16)
-        return launch_pdl(rt, qwen35_rms_norm_kernel<false, true>, dim3(rows), dim3(kNormThreads), "qwen35_rms_norm launch",
+        return launch_pdl(rt, "qwen35_rms_norm launch", qwen35_rms_norm_kernel<false, true>, dim3(rows), dim3(kNormThreads), 0,
                           (const float *)nullptr, xp, wp, out.ptr, dim, eps);
-    return launch_pdl(rt, qwen35_rms_norm_kernel<false, false>, dim3(rows), dim3(kNormThreads), "qwen35_rms_norm launch",
+    return launch_pdl(rt, "qwen35_rms_norm launch", qwen35_rms_norm_kernel<false, false>, dim3(rows), dim3(kNormThreads), 0,
                       (const float *)nullptr, xp, wp, out.ptr, dim, eps);
 }
 
@@ -166,8 +152,7 @@ Result qwen35_residual_add(TesslRuntime *rt, const TesslBuf &y, const TesslBuf &
     const Named writes[] = {{"resid", &resid}};
     const Named reads[] = {{"y", &y}};
     TESSL_TRY(require_disjoint_writes(what, writes, 1, reads, 1));
-    return launch_pdl(rt, qwen35_residual_add_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256),
-                      "qwen35_residual_add launch", static_cast<const float *>(y.ptr), static_cast<float *>(resid.ptr), n);
+    return launch_pdl(rt, "qwen35_residual_add launch", qwen35_residual_add_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, static_cast<const float *>(y.ptr), static_cast<float *>(resid.ptr), n);
 }
 
 Result qwen35_add_rms_norm(TesslRuntime *rt, const TesslBuf &y, const TesslBuf &resid, const TesslBuf &w, const TesslBuf &out,
@@ -190,9 +175,9 @@ Result qwen35_add_rms_norm(TesslRuntime *rt, const TesslBuf &y, const TesslBuf &
     const float *yp = static_cast<const float *>(y.ptr), *wp = static_cast<const float *>(w.ptr);
     float *rp = static_cast<float *>(resid.ptr);
     if (out_as_bf16)
-        return launch_pdl(rt, qwen35_rms_norm_kernel<true, true>, dim3(rows), dim3(kNormThreads), "qwen35_add_rms_norm launch",
+        return launch_pdl(rt, "qwen35_add_rms_norm launch", qwen35_rms_norm_kernel<true, true>, dim3(rows), dim3(kNormThreads), 0,
                           yp, rp, wp, out.ptr, dim, eps);
-    return launch_pdl(rt, qwen35_rms_norm_kernel<true, false>, dim3(rows), dim3(kNormThreads), "qwen35_add_rms_norm launch", yp,
+    return launch_pdl(rt, "qwen35_add_rms_norm launch", qwen35_rms_norm_kernel<true, false>, dim3(rows), dim3(kNormThreads), 0, yp,
                       rp, wp, out.ptr, dim, eps);
 }
 

@@ -97,6 +97,22 @@ inline Result smem_opt_in(TesslRuntime *rt, const void *kernel, size_t bytes, co
     return ok();
 }
 
+/// Launches `kernel` on the runtime's stream with programmatic stream serialization: it may start while the kernel in
+/// front of it drains, so it waits (griddepcontrol.wait) before it touches what that one writes or reads.
+template <typename K, typename... A>
+inline Result launch_pdl(TesslRuntime *rt, const char *what, K kernel, dim3 grid, dim3 block, size_t smem, A... args)
+{
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = grid, lc.blockDim = block, lc.dynamicSmemBytes = smem, lc.stream = rt->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = attr, lc.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&lc, kernel, args...);
+    rt->dispatch_count += 1;
+    return cuda_check(rt, e, what);
+}
+
 /// Scratch of at least `bytes`, 256-byte aligned. Growing waits for the stream
 /// (earlier kernels may still read the old allocation) and reallocates.
 inline Result scratch_reserve(TesslRuntime *rt, size_t bytes, void **out)
