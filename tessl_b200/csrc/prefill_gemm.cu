@@ -481,12 +481,15 @@ Result prefill_validate(const TesslQ4MlxBank &bank, const TesslBuf &x_bf16, cons
 /// at m = 16 .. 64, N = 12288, K = 4096. So the pair kernel runs for every m; the single-CTA kernel is
 /// what a GPU with one SM, or `tessl_runtime_set_prefill_tile(rt, bn, 0)`, selects.
 
-/// Tile width with the least estimated time: waves of tiles x the cost of one tile's K block.
-int pick_tile_width(uint64_t tiles_m, uint32_t n, uint32_t slots)
+/// Tile width with the least estimated time: waves of tiles x the cost of one tile's K block. The 64-wide tile (pair kernel
+/// only) is for calls whose wider tiles leave clusters idle: 77 x 4096 x 12288 is 32 tiles of 128 on 74 clusters, 62.3 us,
+/// and 64 of 64, 53.3 us; 509 x 2048 x 6144 36.9 -> 32.3 us. What is left there is the chain of K blocks, 0.26 us each.
+int pick_tile_width(uint64_t tiles_m, uint32_t n, uint32_t slots, bool pair)
 {
     int best_bn = 256;
     uint64_t best_cost = ~0ull;
-    for (int bn : {256, 192, 128}) {
+    for (int bn : {256, 192, 128, 64}) {
+        if (bn == 64 && !pair) continue;
         const uint64_t tiles = tiles_m * ((n + bn - 1) / bn);
         const uint64_t waves = (tiles + slots - 1) / slots;
         // a K block costs a fixed part (measured: about 320 columns' worth) plus a part proportional to the width
@@ -509,7 +512,7 @@ Result prefill_launch(TesslRuntime *rt, const TesslQ4MlxBank &bank, const TesslB
     const uint32_t tiles_m = pair ? (m + 2 * BM - 1) / (2 * BM) : (m + BM - 1) / BM;
     const int bn = rt->prefill_force_bn
                        ? rt->prefill_force_bn
-                       : pick_tile_width(tiles_m, pl.n, pair ? (uint32_t)rt->sm_count / 2 : (uint32_t)rt->sm_count);
+                       : pick_tile_width(tiles_m, pl.n, pair ? (uint32_t)rt->sm_count / 2 : (uint32_t)rt->sm_count, pair);
     rt->prefill_last_bn = bn, rt->prefill_last_pair = pair ? 1 : 0;
 
     EncodeTiled enc = nullptr;
@@ -535,6 +538,7 @@ Result prefill_launch(TesslRuntime *rt, const TesslQ4MlxBank &bank, const TesslB
     if (pair) {
         if (bn == 256) return launch_gemm_pair<256>(rt, ma, mw, p);
         if (bn == 192) return launch_gemm_pair<192>(rt, ma, mw, p);
+        if (bn == 64) return launch_gemm_pair<64>(rt, ma, mw, p);
         return launch_gemm_pair<128>(rt, ma, mw, p);
     }
     if (bn == 256) return launch_gemm<256>(rt, ma, mw, p);

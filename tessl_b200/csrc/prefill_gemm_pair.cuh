@@ -34,7 +34,7 @@ namespace pf {
 template <int BN>
 struct PairCfg {
     static constexpr int HB = BN / 2;                 // weight rows this CTA expands
-    static constexpr int SA = 6;                      // stages of the (X tile, dequantized-W tile) ring
+    static constexpr int SA = BN == 64 ? 10 : 6;      // stages of the (X tile, dequantized-W tile) ring
     static constexpr int SB = SA;                     // one ring: a K block's two operands are freed together
     static constexpr int SQ = BN == 256 ? 4 : 8;      // packed-W stages
     static constexpr int NDW = HB / 16;               // dequant warps per group (two threads per weight row)
