@@ -324,7 +324,6 @@ __global__ void __launch_bounds__(Cfg<BN>::THREADS, 1)
             for (uint32_t c = 0; c < BN / 32; ++c) {
                 uint32_t r[32];
                 tmem_ld32(tmem_base + ((quarter * 32u) << 16) + buf * 256u + c * 32u, r);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 store_row32(p, r, m, n0 + c * 32, rs);
             }
             tcgen05_fence_before();

@@ -234,7 +234,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<BN>::THREADS
             for (uint32_t c = 0; c < BN / 32; ++c) {
                 uint32_t r[32];
                 tmem_ld32(tmem_base + ((quarter * 32u) << 16) + buf * 256u + c * 32u, r);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 store_block32_coalesced(p, r, stage, lane, m_base, n0 + c * 32, rs);
             }
             tcgen05_fence_before();
