@@ -54,8 +54,8 @@ struct TesslRuntime {
     // alias) when a bounded wait inside it gives up. Checked at every wait.
     volatile uint32_t *status_host = nullptr;
     uint32_t *status_dev = nullptr;
-    // Dynamic shared memory already opted in, per kernel. The attribute belongs to the
-    // device's context, so it is remembered per runtime (one device each), not per process.
+    // Dynamic shared memory a block of a kernel may have, per kernel that was opted in. The attribute belongs to
+    // the device's context, so it is remembered per runtime (one device each), not per process.
     std::map<const void *, size_t> smem_opted;
     // Clusters of a given size that the device holds at once, per kernel (asked once).
     std::map<std::pair<const void *, uint32_t>, int> max_clusters;
@@ -80,20 +80,31 @@ inline Result cuda_check(TesslRuntime *rt, cudaError_t e, const char *what)
                cudaGetErrorString(e));
 }
 
-/// Opts `kernel` in to `bytes` of dynamic shared memory on the runtime's device, once per
-/// runtime and size; `carveout` also asks for the largest shared-memory carve-out.
+/// Makes sure that `kernel` may be launched with `bytes` of dynamic shared memory; `carveout` also asks for the largest
+/// shared-memory carve-out. The limit belongs to the device's context, which all runtimes of the device share, and one
+/// kernel serves launches of many sizes: so every runtime sets the same value, all that a block of the kernel may have.
+/// (Set to the launch's own size, one runtime lowered it under another, whose next launch failed.)
 inline Result smem_opt_in(TesslRuntime *rt, const void *kernel, size_t bytes, const char *what, bool carveout = false)
 {
     auto it = rt->smem_opted.find(kernel);
-    if (it != rt->smem_opted.end() && it->second >= bytes) return ok();
-    Result r = cuda_check(rt, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), what);
-    if (!r.empty()) return r;
-    if (carveout) {
-        r = cuda_check(rt, cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                                (int)cudaSharedmemCarveoutMaxShared), what);
+    if (it == rt->smem_opted.end()) {
+        int optin = 0;
+        cudaFuncAttributes fa{};
+        Result r = cuda_check(rt, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, rt->device), what);
         if (!r.empty()) return r;
+        r = cuda_check(rt, cudaFuncGetAttributes(&fa, kernel), what);
+        if (!r.empty()) return r;
+        const size_t limit = (size_t)optin - fa.sharedSizeBytes;
+        r = cuda_check(rt, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit), what);
+        if (!r.empty()) return r;
+        if (carveout) {
+            r = cuda_check(rt, cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                                    (int)cudaSharedmemCarveoutMaxShared), what);
+            if (!r.empty()) return r;
+        }
+        it = rt->smem_opted.emplace(kernel, limit).first;
     }
-    rt->smem_opted[kernel] = bytes;
+    if (bytes > it->second) return fmt("%s: a block would need %zu bytes, the device has %zu", what, bytes, it->second);
     return ok();
 }
 
