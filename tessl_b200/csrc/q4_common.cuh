@@ -51,16 +51,23 @@ __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w 
 
 /// Power-of-two scaling of a slice of bf16 activations that meets nibbles held as bf16 subnormals (q * 2^-133): `mul` =
 /// (2^e, 2^e) and `mul16` = (2^(e-4), 2^(e-4)) as bf16 pairs, `undo` = 2^(133-e). e brings the slice's largest magnitude
-/// to about 2^100, so that every product is a normal f32, within what a bf16 factor (e <= 127) and an f32 undo (e >= 6)
-/// can hold. The affine fold of the slice then runs in units of `undo` (`scaled_sum`: a group sum in those units): the
-/// same roundings as on the plain values, without a multiplication per dot product. `amax`: the largest magnitude's bits.
+/// to 2^126, as far as a bf16 factor (e <= 127) and an f32 undo (e >= 6) can. The affine fold of the slice then runs in
+/// units of `undo` (`scaled_sum`: a group sum in those units), without a multiplication per dot product, and rounds as
+/// the plain values do wherever nothing leaves the range:
+///   * `undo` >= 2^6, so no sum overflows before the plain one would;
+///   * it is the smallest unit that can be had (2^6, or 2^7 times the slice's largest power of two), so the fold reaches
+///     the f32 subnormals only with scales below 2^-122 (the smallest normal bf16 is 2^-126), or results below 2^-120. With the
+///     slice brought to 2^100 only, scales below 2^-93 lost their bits;
+///   * products are multiples of 2^-149 as long as the slice's largest magnitude is below 2^10, subnormal activations
+///     included, so the tensor cores lose none; above, those over 2^135 times smaller than the largest lose bits;
+///   * from 2^122 on a scaled activation overflows: Inf or NaN results, as from f32 sums of a group of such activations.
 struct XScale {
     uint32_t mul, mul16;
     float undo, sum1;
 };
 __device__ __forceinline__ XScale x_scale(uint32_t amax)
 {
-    const int e = min(127, max(6, 100 + 127 - (int)(amax >> 7)));
+    const int e = min(127, max(6, 126 + 127 - (int)(amax >> 7)));
     return XScale{(uint32_t)(e + 127) * 0x00800080u, (uint32_t)(e + 123) * 0x00800080u, __uint_as_float((uint32_t)(127 + 133 - e) << 23),
                   __uint_as_float((uint32_t)(e + 57) << 23)};
 }
@@ -73,7 +80,7 @@ __device__ __forceinline__ uint32_t bf2_mul(uint32_t a, uint32_t b)
     return r;
 }
 /// Eight activations -> the B registers of the two MMAs that take the eight nibbles of a packed word:
-/// (x0, x4), (x1, x5) / 16, (x2, x6), (x3, x7) / 16, scaled. Exact: only exponents change.
+/// (x0, x4), (x1, x5) / 16, (x2, x6), (x3, x7) / 16, scaled. Only exponents change (within the bounds above).
 __device__ __forceinline__ void x_fragment(const uint4 &v, const XScale &s, uint32_t (&f)[4])
 {
     f[0] = bf2_mul(__byte_perm(v.x, v.z, 0x5410), s.mul), f[1] = bf2_mul(__byte_perm(v.x, v.z, 0x7632), s.mul16);

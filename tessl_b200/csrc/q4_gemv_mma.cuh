@@ -588,9 +588,8 @@ __global__ void __launch_bounds__(kThreads, TESSL_GEMV_MMA_MIN_BLOCKS) q4_gemv_m
         float xs[NGS];  // group sums of the activations: column g (BATCH) or the vector (M = 1)
         // Q4: the nibbles go to the MMA as the bf16 bit patterns 0..15 and 16 x (0..15), i.e. q * 2^-133 (the
         // subnormal range and the first binade of bf16 are one linear scale), so the activations carry the
-        // rest: times 2^e (e puts the slice's largest magnitude of this row of x near 2^100, so that every
-        // product is a normal f32), the partners of the odd nibbles divided by 16 as well. Both are changes
-        // of the exponent field only, hence exact; `cw` = 2^(133 - e) undoes them in the fold.
+        // rest: times 2^e (from the slice's largest magnitude of this row of x, see dev::x_scale), the partners of
+        // the odd nibbles divided by 16 as well; `cw` = 2^(133 - e) undoes them in the fold.
         float cw = 0.0f;
         float cwv[NWIN];  // per window (M = 1)
         // this lane's B fragments and group sums of window `win`, from the warp's staged copy
