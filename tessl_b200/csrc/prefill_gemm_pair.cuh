@@ -39,6 +39,9 @@ struct PairCfg {
     static constexpr int SQ = BN == 256 ? 4 : 8;      // packed-W stages
     static constexpr int NDW = HB / 16;               // dequant warps per group (two threads per weight row)
     static constexpr int NG = 2;                      // dequant groups; group g expands K blocks g, g + 2, ...
+    // A group starts every tile at block g, so its step across the end of a tile is up to 2 NG - 1 blocks; a step longer
+    // than its ring would make the parity that it waits for ambiguous.
+    static_assert(2 * NG - 1 <= SA && 2 * NG - 1 <= SQ, "a dequant group may step past a whole ring");
     static constexpr int FIRST_DW = 8;                // first dequant warp
     static constexpr int THREADS = (FIRST_DW + NG * NDW) * 32;
     // Sleep between mbarrier polls (ns) of the roles that run ahead of the MMA issuer.
