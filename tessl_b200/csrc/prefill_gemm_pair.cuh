@@ -64,7 +64,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<BN>::THREADS
                                 const GemmParams p)
 {
     using C = PairCfg<BN>;
-    asm volatile("griddepcontrol.launch_dependents;");
+    // No early start for the launch behind this one: it is often the next projection's pre-pass, whose blocks would settle on the
+    // few SMs that this grid leaves idle and convert their rows there, unevenly. 257 x 4096 x 12288 72.9 us with a trigger here,
+    // 68.2 without, 509 x 2048 x 6144 34.1 / 31.9, a layer over 509 rows of 2048 134.5 / 124.3; the smallest calls miss the
+    // overlap (257 x 1024 x 1024 10.1 / 10.9).
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
@@ -122,7 +125,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<BN>::THREADS
     if (warp == 0) {
         // ------------------------------------------------ TMA producer: X tiles ---
         if (lane == 0) {
-            asm volatile("griddepcontrol.wait;" ::: "memory");  // the pre-pass writes the activations
+            // The pre-pass writes the activations with ordinary stores, the copies below read them through the async proxy. The end
+            // of a kernel orders the two; the wait of a programmatic launch promises that for ordinary loads only.
+            asm volatile("griddepcontrol.wait;\n\tfence.proxy.async.global;" ::: "memory");
             RingPos<C::SA> ring;
             bool ok_ = true;
             for (uint32_t t = cluster_id; t < ntiles && ok_; t += nclusters) {
