@@ -503,10 +503,10 @@ bool batch_ok(const Q4GemvParams &p, int m, int nb)
     return batch_plan(p.cols, p.group_shift).ngs != 0;
 }
 
-template <int WPG, int NGS, bool EVEN, int NB>
+template <int WPG, int NGS, bool EVEN, int NB, bool ONE>
 Result launch_batch_one(TesslRuntime *rt, const Q4GemvParams &p, int m, const BatchPlan &b)
 {
-    auto kernel = q4b::q4_batch_mma_kernel<WPG, NGS, EVEN, NB>;
+    auto kernel = q4b::q4_batch_mma_kernel<WPG, NGS, EVEN, NB, ONE>;
     constexpr uint32_t RPB = q4b::kRows / NB;
     const char *what = "q4_gemv";
     EncodeTiled enc = nullptr;
@@ -562,7 +562,7 @@ Result launch_batch_one(TesslRuntime *rt, const Q4GemvParams &p, int m, const Ba
                 n = std::max(1, rt->sm_count / (int)b.nwin);
             }
         }
-        clusters = (uint32_t)n; 
+        clusters = (uint32_t)n;
     }
     clusters = std::min(clusters, bp.total_rb);
     const uint64_t step = (((uint64_t)bp.total_rb << 32) + clusters - 1) / clusters;
@@ -579,11 +579,12 @@ Result launch_batch_ngs(TesslRuntime *rt, const Q4GemvParams &p, int m, int nb, 
     if constexpr (NGS > 1) {
         if (b.ngs != NGS) return launch_batch_ngs<WPG, NGS - 1>(rt, p, m, nb, b);
     }
-    if (nb == 2) return launch_batch_one<WPG, NGS, false, 2>(rt, p, m, b);
+    if (nb == 2) return launch_batch_one<WPG, NGS, false, 2, true>(rt, p, m, b);
+    if (m == 1) return launch_batch_one<WPG, NGS, false, 1, true>(rt, p, m, b);
     if constexpr ((NGS & (NGS - 1)) == 0) {
-        if (b.even) return launch_batch_one<WPG, NGS, true, 1>(rt, p, m, b);
+        if (b.even) return launch_batch_one<WPG, NGS, true, 1, false>(rt, p, m, b);
     }
-    return launch_batch_one<WPG, NGS, false, 1>(rt, p, m, b);
+    return launch_batch_one<WPG, NGS, false, 1, false>(rt, p, m, b);
 }
 
 Result launch_batch(TesslRuntime *rt, const Q4GemvParams &p, int m, int nb)
@@ -682,10 +683,12 @@ Result launch_q4_gemv(TesslRuntime *rt, Q4GemvParams p, int m, int nb)
         if (p.peer) return nn::peer_gather(rt, *static_cast<const TesslPeerGather *>(p.peer));
         return ok();
     }
-    // One row of x over shorter rows leaves most of the 16 consumer warps without a group: 60000 x 512 8.9 us on the FMA
-    // pipe against 12.5 here, 4096 x 512 2.33 / 2.48; from 1024 columns on 1024 x 1280 2.61 / 2.27, 6144 x 2560 5.50 / 4.26,
-    // 2048 x 6144 4.72 / 4.85, 2560 x 9216 7.55 / 6.70, 4096 x 17408 24.6 / 12.3, 40000 x 6144 35.4 / 26.2. A function of K
-    // alone, so that a row's summation order stays one of K and G.
+    // One row of x over shorter rows leaves most of the 16 consumer warps without a group: 60000 x 512 8.8 us on the FMA
+    // pipe against 12.0 here, 4096 x 512 2.32 / 2.34; from 1024 columns on 1024 x 1280 2.60 / 1.87, 6144 x 2560 5.55 / 3.72,
+    // 2048 x 6144 4.81 / 4.38, 2560 x 9216 7.89 / 6.01, 4096 x 17408 24.6 / 10.4, 40000 x 6144 35.8 / 23.1, gate/up 13824 x 5120
+    // 25.0 / 21.4, 2048 x 6144 6.41 / 6.46. Few rows over the windows of a cluster pay its fixed part: 257 x 7168 2.76 / 2.92,
+    // 1024 x 9216 4.46 / 4.51 (groups of 128: 4.41 / 4.86), gate/up 512 x 9216 4.00 / 4.71. The line is one of K alone all the
+    // same, so that a row's summation order is one of K and G (fused and separate launches, slices of a bank).
     if (m == 1 && p.cols >= 1024 && batch_ok(p, m, nb)) return launch_batch(rt, p, m, nb);
     if (m == 1 && nchunks <= 4 && tma_ok(p)) {
         if (nb == 1) {
@@ -1104,9 +1107,9 @@ Result swiglu(TesslRuntime *rt, const TesslBuf &gate, const TesslBuf &up, const 
 }
 
 /// A validated prefill call with few rows, run as batches of up to 8 rows on the tensor-core GEMV kernel:
-/// up to 24 rows that is faster than the prefill GEMM, whose 256-row tile would be mostly padding
-/// (12288 x 4096: 9.3 us per batch of 8 against 34.6 us for any m <= 64). `*handled` is false when the shape
-/// is not one that kernel is built for.
+/// up to 24 rows that is faster than the prefill GEMM, whose 256-row tile would be mostly padding (24 rows as three
+/// batches against 25 through the GEMM: 12288 x 4096 23.8 / 33.2 us, 4096 x 4096 13.9 / 22.0, 2048 x 2048 8.1 / 13.3, 1024 x
+/// 1024 6.7 / 9.7). At the widths where a single row has the tensor-core kernel; `*handled` is false at the others.
 Result prefill_as_small_batches(TesslRuntime *rt, const TesslQ4MlxBank &bank, const TesslBuf &x_bf16, const TesslBuf &y,
                                 const TesslQuantShape &shape, uint32_t m, OutKind out, bool *handled)
 {

@@ -78,3 +78,18 @@ def test_fused_single_row_forms_equal_separate_launches(rt, rows, cols, group):
     nn.swiglu(rt, outs[0], outs[1], want, rows, False)
     v = mid.read(np.float32, rows + 8)
     assert np.array_equal(v[:rows].view(np.uint32), want.read(np.uint32, rows)) and np.all(v[rows:] == SENTINEL_F32)
+
+
+@pytest.mark.parametrize("rows,cols,group", [(40, 1024, 64), (40, 2048, 32), (40, 4096, 128), (40, 2560, 64), (17, 3840, 32), (33, 9216, 64),
+                                             (16, 17408, 64), (20, 12800, 128)])
+def test_a_batch_row_equals_the_vector_alone(rt, rows, cols, group):
+    """Bit for bit at 1024, 2048 and 4096 columns (the single-row kernel sums in the same order) and where one row runs on
+    the batch kernel itself."""
+    bank, shape = upload_bank(rt, *synth.q4_bank(0x7E551700 + cols, rows, cols, group)), nn.QuantShape(rows, cols, group)
+    x = synth.normal_bf16(0x7E551710 + cols, 8 * cols)
+    y8, y1 = seeded_f32(rt, 8 * rows), seeded_f32(rt, rows)
+    nn.gemm_q4_mlx(rt, bank, rt.buffer_from(x), y8, shape, 8)
+    got = y8.read(np.uint32, 8 * rows).reshape(8, rows)
+    for i in (0, 5, 7):
+        nn.gemv_q4_mlx_simd(rt, bank, rt.buffer_from(x[i * cols:(i + 1) * cols].copy()), y1, shape)
+        assert np.array_equal(y1.read(np.uint32, rows), got[i])
