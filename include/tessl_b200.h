@@ -129,9 +129,9 @@ TESSL_API int32_t tessl_runtime_device(TesslRuntime *rt);
 TESSL_API int32_t tessl_runtime_poison_for_test(TesslRuntime *rt);
 
 /* Prefill GEMM tile choice, for tuning runs and for tests that must reach every
- * compiled tile: tile_n in {128, 192, 256} forces the tile width of later
+ * compiled tile: tile_n in {64, 128, 192, 256} forces the tile width of later
  * tessl_gemm_q4_mlx_tensorops* calls on this runtime (0 = the library's own
- * estimate), pair = 1 / 0 forces the two-CTA or the single-CTA kernel (-1 = the
+ * estimate; 64 with pair = 1 only), pair = 1 / 0 forces the two-CTA or the single-CTA kernel (-1 = the
  * library decides). tessl_runtime_last_prefill_tile reports what the most
  * recent prefill call launched (tile_n = 0 if it ran no tile kernel). No
  * counterpart in the reference, whose kernel has one 32 x 32 tile. */

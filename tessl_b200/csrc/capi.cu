@@ -247,10 +247,14 @@ int32_t tessl_runtime_poison_for_test(TesslRuntime *rt)
 int32_t tessl_runtime_set_prefill_tile(TesslRuntime *rt, uint32_t tile_n, int32_t pair, char *err, size_t err_len)
 {
     if (refuse_unowned(rt, err, err_len)) return TESSL_ERR;
-    if ((tile_n != 0 && tile_n != 128 && tile_n != 192 && tile_n != 256) || pair < -1 || pair > 1) {
+    if ((tile_n != 0 && tile_n != 64 && tile_n != 128 && tile_n != 192 && tile_n != 256) || pair < -1 || pair > 1) {
         write_err(err, err_len,
-                  tessl::fmt("tessl_runtime_set_prefill_tile: tile_n %u is not one of [0, 128, 192, 256] or pair %d is "
+                  tessl::fmt("tessl_runtime_set_prefill_tile: tile_n %u is not one of [0, 64, 128, 192, 256] or pair %d is "
                              "not one of [-1, 0, 1]", tile_n, pair));
+        return TESSL_ERR;
+    }
+    if (tile_n == 64 && pair != 1) {
+        write_err(err, err_len, tessl::fmt("tessl_runtime_set_prefill_tile: the 64-wide tile exists in the two-CTA kernel only (pair = 1, got %d)", pair));
         return TESSL_ERR;
     }
     rt->prefill_force_bn = (int)tile_n;

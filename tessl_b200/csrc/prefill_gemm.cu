@@ -537,9 +537,10 @@ Result prefill_launch(TesslRuntime *rt, const TesslQ4MlxBank &bank, const TesslB
     if (pair) {
         if (bn == 256) return launch_gemm_pair<256>(rt, ma, mw, p);
         if (bn == 192) return launch_gemm_pair<192>(rt, ma, mw, p);
-        if (bn == 64) return launch_gemm_pair<64>(rt, ma, mw, p);
-        return launch_gemm_pair<128>(rt, ma, mw, p);
+        if (bn == 128) return launch_gemm_pair<128>(rt, ma, mw, p);
+        return launch_gemm_pair<64>(rt, ma, mw, p);
     }
+    if (bn == 64) return fmt("%s: the 64-wide tile exists in the two-CTA kernel only", kWhat);
     if (bn == 256) return launch_gemm<256>(rt, ma, mw, p);
     if (bn == 192) return launch_gemm<192>(rt, ma, mw, p);
     return launch_gemm<128>(rt, ma, mw, p);

@@ -174,7 +174,7 @@ class Runtime:
         return out.value
 
     def set_prefill_tile(self, tile_n: int = 0, pair: int = -1) -> None:
-        """Force the prefill GEMM's tile width (128 / 192 / 256, 0 = automatic) and kernel
+        """Force the prefill GEMM's tile width (64 with the CTA pair, 128 / 192 / 256, 0 = automatic) and kernel
         (1 = CTA pair, 0 = single CTA, -1 = automatic) for later calls on this runtime."""
         capi.call("tessl_runtime_set_prefill_tile", self.handle, tile_n, pair)
 
