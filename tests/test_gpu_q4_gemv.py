@@ -170,17 +170,17 @@ def test_small_m_gemm_matches_the_oracle(rt, rows, cols, group, m):
 
 TENSOR_GEMV_SHAPES = [(40, 1024, 32), (257, 1024, 64), (40, 2048, 32), (257, 2048, 64), (72, 2048, 128),
                       (40, 4096, 32), (129, 4096, 64), (257, 4096, 128),
-                      # longer rows: M = 1 on the FMA-pipe kernels, batches as windows of 4096 columns on
-                      # the MMA kernel, each launch adding to the ones before it; same contract
+                      # longer rows: M = 1 over 8192 and 12288 columns on the single-row kernel's windows, the
+                      # others and all batches on the batch kernel's (csrc/q4_batch_mma.cuh); same contract
                       (40, 8192, 64), (257, 12288, 64), (72, 8192, 128), (33, 16384, 32),
-                      (40, 6144, 64)]  # not a multiple of 4096: FMA-pipe kernels for every M
+                      (40, 6144, 64)]
 
 
 @pytest.mark.parametrize("rows,cols,group", TENSOR_GEMV_SHAPES)
 def test_tensor_core_gemv_shapes(rt, rows, cols, group):
-    """Rows of 1024, 2048 or 4096 columns run on the MMA kernel: every (K, G) it is built
-    for, ragged row counts, batches of 1, 3 and 8, and the fused gate/up launch against
-    two plain launches."""
+    """The widths of the single-row tensor-core kernel (every (K, G) it is built for) and some of the batch
+    kernel's: ragged row counts, batches of 1, 3 and 8, and the fused gate/up launch against two plain
+    launches."""
     packed, sb, _ = make_case(rows, cols, group, 0x7E550090 + rows + cols)
     bank = upload_bank(rt, packed, sb)
     shape = nn.QuantShape(rows, cols, group)
