@@ -482,7 +482,7 @@ Result prefill_validate(const TesslQ4MlxBank &bank, const TesslBuf &x_bf16, cons
 
 /// Tile width with the least estimated time: waves of tiles x the cost of one tile's K block. The 64-wide tile (pair kernel
 /// only) is for calls whose wider tiles leave clusters idle: 77 x 4096 x 12288 is 32 tiles of 128 on 74 clusters, 62.3 us,
-/// and 64 of 64, 53.3 us; 509 x 2048 x 6144 36.9 -> 32.3 us. What is left there is the chain of K blocks, 0.26 us each.
+/// and 64 of 64, 52.7 us; 509 x 2048 x 6144 35.7 / 30.2 us, 257 x 1024 x 1024 10.3 / 9.1. What is left there is the chain of K blocks, 0.26 us each.
 int pick_tile_width(uint64_t tiles_m, uint32_t n, uint32_t slots, bool pair)
 {
     int best_bn = 256;
