@@ -13,12 +13,14 @@ namespace pf {
 
 using q4k::and_or;
 using q4k::lds128;
+using q4k::map_to_cta;
 using q4k::mbar_arrive;
 using q4k::mbar_expect_tx;
 using q4k::mbar_init;
 using q4k::mbar_try;
 using q4k::mbar_wait;
 using q4k::smem_u32;
+using q4k::tma_load_2d;
 
 constexpr int BM = 128;  // rows of X per tile = MMA M
 constexpr int BK = 64;   // K block: 128 bytes of f16 = one swizzle row
@@ -41,14 +43,6 @@ struct GemmParams {
 
 // ---------------------------------------------------------------- PTX wrappers ---
 
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-            dst),
-        "l"(map), "r"(x), "r"(y), "r"(bar)
-        : "memory");
-}
 __device__ __forceinline__ void tcgen05_commit(uint32_t bar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -282,13 +276,6 @@ __device__ __forceinline__ uint32_t cluster_ctarank()
 {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-/// The shared::cluster address of `local_addr` (a shared::cta address) in CTA `rank` of this cluster.
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t local_addr, uint32_t rank)
-{
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank));
     return r;
 }
 __device__ __forceinline__ void cluster_sync_all()

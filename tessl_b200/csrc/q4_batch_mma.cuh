@@ -39,12 +39,14 @@ namespace tessl {
 namespace q4b {
 
 using q4k::lds32;
+using q4k::map_to_cta;
 using q4k::mbar_arrive;
 using q4k::mbar_expect_tx;
 using q4k::mbar_init;
 using q4k::mbar_try;
 using q4k::mbar_wait;
 using q4k::smem_u32;
+using q4k::tma_load_2d;
 using q4m::lds64;
 using q4m::mma_bf16;
 
@@ -92,18 +94,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map
         "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
         "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
         : "memory");
-}
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar)
-{
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-                 "l"(map), "r"(x), "r"(y), "r"(bar)
-                 : "memory");
-}
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t local_addr, uint32_t rank)
-{
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank));
-    return r;
 }
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr)
 {

@@ -21,6 +21,8 @@
 // loop, gives the copies it requested a bounded chance to land, and returns.
 #pragma once
 
+#include <cuda.h>
+
 #include "q4_gemv_kernel.cuh"
 
 namespace tessl {
@@ -51,6 +53,13 @@ struct TmaParams {
     uint32_t *status;  // runtime status word (pinned host memory), written only on a timeout
 };
 
+/// The shared::cluster address of `local_addr` (a shared::cta address) in CTA `rank` of this cluster.
+__device__ __forceinline__ uint32_t map_to_cta(uint32_t local_addr, uint32_t rank)
+{
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank));
+    return r;
+}
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
@@ -102,6 +111,16 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
                  "l"(src), "r"(bytes), "r"(bar)
                  : "memory");
+}
+
+/// A tile of a 2-D tensor map; completes on `bar`.
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+            dst),
+        "l"(map), "r"(x), "r"(y), "r"(bar)
+        : "memory");
 }
 __device__ __forceinline__ uint4 lds128(uint32_t addr)
 {
