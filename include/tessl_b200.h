@@ -133,7 +133,9 @@ TESSL_API int32_t tessl_runtime_poison_for_test(TesslRuntime *rt);
  * tessl_gemm_q4_mlx_tensorops* calls on this runtime (0 = the library's own
  * estimate; 64 with pair = 1 only), pair = 1 / 0 forces the two-CTA or the single-CTA kernel (-1 = the
  * library decides). tessl_runtime_last_prefill_tile reports what the most
- * recent prefill call launched (tile_n = 0 if it ran no tile kernel). No
+ * recent prefill call launched (tile_n = 0 if it ran no tile kernel; 64 with
+ * pair = 1 stands for the narrow ones: the 64-wide tile, and the kernel that
+ * divides K over a cluster, which the library alone chooses). No
  * counterpart in the reference, whose kernel has one 32 x 32 tile. */
 TESSL_API int32_t tessl_runtime_set_prefill_tile(TesslRuntime *rt, uint32_t tile_n, int32_t pair, char *err, size_t err_len);
 TESSL_API int32_t tessl_runtime_last_prefill_tile(TesslRuntime *rt, uint32_t *tile_n, uint32_t *pair, char *err,

@@ -21,6 +21,7 @@ using q4k::mbar_try;
 using q4k::mbar_wait;
 using q4k::smem_u32;
 using q4k::tma_load_2d;
+using q4k::tma_load_3d;
 
 constexpr int BM = 128;  // rows of X per tile = MMA M
 constexpr int BK = 64;   // K block: 128 bytes of f16 = one swizzle row
@@ -111,29 +112,34 @@ __device__ __forceinline__ uint32_t pack_h2(__half lo, __half hi)
 
 // ------------------------------------------------- weight expansion, stores ---
 
-/// NW packed words (8 nibbles each) of one weight row -> 8 NW f16 values
-/// s * (q - 8), written as 16-byte chunks c0 .. c0 + NW - 1 of the 128-byte row at
-/// `brow` with the 128B swizzle (`swz` = (row & 7) << 4). `s` is the group scale
-/// as an f16 pair. Each chunk holds the eight weights of one packed word in the
-/// order 0,4,1,5,2,6,3,7.
+/// One packed word (8 nibbles) -> 8 f16 values s * (q - 8) in the order 0,4,1,5,2,6,3,7. `s` is the group scale as an
+/// f16 pair.
+__device__ __forceinline__ void expand_q4_word(uint32_t w, uint32_t s, uint32_t *o)
+{
+    const uint32_t w8 = w >> 8;
+    // (1024 + q) and (1024 + 16 q) as f16 pairs, then q - 8 exactly, then * s exactly
+    const uint32_t t0 = and_or(w, 0x000f000fu, 0x64006400u);
+    const uint32_t t1 = and_or(w, 0x00f000f0u, 0x64006400u);
+    const uint32_t t2 = and_or(w8, 0x000f000fu, 0x64006400u);
+    const uint32_t t3 = and_or(w8, 0x00f000f0u, 0x64006400u);
+    o[0] = h2_mul(h2_sub(t0, 0x64086408u), s);               // 1024 + q - 1032
+    o[1] = h2_mul(h2_fma(t1, 0x2c002c00u, 0xd480d480u), s);  // (1024 + 16 q) / 16 - 72
+    o[2] = h2_mul(h2_sub(t2, 0x64086408u), s);
+    o[3] = h2_mul(h2_fma(t3, 0x2c002c00u, 0xd480d480u), s);
+}
+
+/// NW packed words of one weight row -> 8 NW f16 values s * (q - 8), written as 16-byte chunks c0 .. c0 + NW - 1 of the
+/// 128-byte row at `brow` with the 128B swizzle (`swz` = (row & 7) << 4), each chunk one word in expand_q4_word's order.
 template <int NW>
 __device__ __forceinline__ void expand_q4_words(const uint32_t (&words)[NW], uint32_t s, uint32_t brow, uint32_t swz,
                                                 uint32_t c0)
 {
 #pragma unroll
     for (int c = 0; c < NW; ++c) {
-        const uint32_t w = words[c], w8 = w >> 8;
-        // (1024 + q) and (1024 + 16 q) as f16 pairs, then q - 8 exactly, then * s exactly
-        const uint32_t t0 = and_or(w, 0x000f000fu, 0x64006400u);
-        const uint32_t t1 = and_or(w, 0x00f000f0u, 0x64006400u);
-        const uint32_t t2 = and_or(w8, 0x000f000fu, 0x64006400u);
-        const uint32_t t3 = and_or(w8, 0x00f000f0u, 0x64006400u);
-        const uint32_t ox = h2_mul(h2_sub(t0, 0x64086408u), s);                // 1024 + q - 1032
-        const uint32_t oy = h2_mul(h2_fma(t1, 0x2c002c00u, 0xd480d480u), s);  // (1024 + 16 q) / 16 - 72
-        const uint32_t oz = h2_mul(h2_sub(t2, 0x64086408u), s);
-        const uint32_t ow = h2_mul(h2_fma(t3, 0x2c002c00u, 0xd480d480u), s);
-        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(brow + (((c0 + (uint32_t)c) << 4) ^ swz)), "r"(ox),
-                     "r"(oy), "r"(oz), "r"(ow)
+        uint32_t o[4];
+        expand_q4_word(words[c], s, o);
+        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(brow + (((c0 + (uint32_t)c) << 4) ^ swz)), "r"(o[0]),
+                     "r"(o[1]), "r"(o[2]), "r"(o[3])
                      : "memory");
     }
 }
@@ -145,9 +151,17 @@ __device__ __forceinline__ uint32_t scale_h2(uint32_t pair)
     return pack_h2(sh, sh);
 }
 
-/// Chunks c0 .. c0 + NC - 1 of extra K block `e` of one weight row: per group
-/// (c1, c1, c1, c2) with c1 + c2 the two-piece f16 split of b + 8 s, two groups
-/// per chunk; groups past `gpr` are zero.
+/// The four extra columns of a group with this (scale, bias) word: (c1, c1), (c1, c2) with c1 + c2 the two-piece f16 split
+/// of b + 8 s. Zeros for a word of zeros (a group past the last).
+__device__ __forceinline__ void extra_pair(uint32_t pair, uint32_t &lo, uint32_t &hi)
+{
+    const float bp = fmaf(8.0f, dev::bf16_lo(pair), dev::bf16_hi(pair));
+    const __half c1 = __float2half_rn(bp);
+    const __half c2 = __float2half_rn(bp - __half2float(c1));
+    lo = pack_h2(c1, c1), hi = pack_h2(c1, c2);
+}
+
+/// Chunks c0 .. c0 + NC - 1 of extra K block `e` of one weight row, two groups per chunk.
 template <int NC>
 __device__ __forceinline__ void expand_extra_chunks(const uint32_t *sbrow, uint32_t e, uint32_t gpr, uint32_t brow,
                                                     uint32_t swz, uint32_t c0)
@@ -159,15 +173,7 @@ __device__ __forceinline__ void expand_extra_chunks(const uint32_t *sbrow, uint3
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             const uint32_t g = e * 16 + 2 * c + j;
-            uint32_t lo = 0, hi = 0;
-            if (g < gpr) {
-                const uint32_t pair = __ldg(sbrow + g);
-                const float bp = fmaf(8.0f, dev::bf16_lo(pair), dev::bf16_hi(pair));
-                const __half c1 = __float2half_rn(bp);
-                const __half c2 = __float2half_rn(bp - __half2float(c1));
-                lo = pack_h2(c1, c1), hi = pack_h2(c1, c2);
-            }
-            o[2 * j] = lo, o[2 * j + 1] = hi;
+            extra_pair(g < gpr ? __ldg(sbrow + g) : 0u, o[2 * j], o[2 * j + 1]);
         }
         asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(brow + ((c << 4) ^ swz)), "r"(o[0]), "r"(o[1]), "r"(o[2]),
                      "r"(o[3])

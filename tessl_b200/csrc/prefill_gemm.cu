@@ -49,6 +49,7 @@
 
 #include "prefill_common.cuh"
 #include "prefill_gemm_pair.cuh"
+#include "prefill_gemm_split.cuh"
 #include "tensormap.h"
 
 namespace tessl {
@@ -65,71 +66,72 @@ using nn::OUT_BF16;
 /// every 8-chunk in the order 0,4,1,5,2,6,3,7 that the nibble-pair dequant
 /// produces on the B side), then the per-group sums as (h1, h2, h3, h1) f16
 /// quadruples, then zero padding. a_aug is [M, K_aug] row-major.
-__global__ void __launch_bounds__(256) x_prepare_kernel(const uint16_t *x, __half *a_aug, float *row_scale, uint32_t K,
-                                                        uint32_t K64, uint32_t K_aug, uint32_t gshift)
+///
+/// A thread holds its NC chunks of 8 elements in registers between the two passes, and the block is as wide as the row asks for:
+/// one round trip to memory and one barrier per row. (256 threads that read the row twice, in steps: 77 rows of 12288
+/// 4.4 us, of 1024 1.9 us.) NC = 0: rows too long for that, read twice.
+constexpr uint32_t kPrepMaxThreads = 768;
+
+template <int NC>
+__global__ void __launch_bounds__(kPrepMaxThreads) x_prepare_kernel(const uint16_t *x, __half *a_aug, float *row_scale, uint32_t K,
+                                                                    uint32_t K64, uint32_t K_aug, uint32_t gshift)
 {
     // Wait first, then let the GEMM start: its blocks set themselves up and stream weights while these rows are converted,
     // and everything in front of this kernel is complete when they do (2 - 4 us per call).
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const uint32_t m = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t m = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = blockDim.x;
     const uint16_t *xrow = x + (size_t)m * K;
     __half *arow = a_aug + (size_t)m * K_aug;
-    __shared__ uint32_t red[8];
-    __shared__ float s_down;
+    __shared__ uint32_t red[kPrepMaxThreads / 32];
 
-    // pass 1: largest magnitude (bf16 bit patterns order like integers); Inf/NaN disable the rescale
+    // largest magnitude (bf16 bit patterns order like integers); Inf/NaN disable the rescale
+    constexpr int HELD = NC > 0 ? NC : 1;
+    uint4 held[HELD];
     uint32_t amax = 0;
-    for (uint32_t ch = tid; ch < K / 8; ch += 256) {
-        const uint4 v = dev::ld_after_wait16(reinterpret_cast<const uint4 *>(xrow) + ch);
+    auto load = [&](uint32_t ch) {
+        return ch * 8 < K ? dev::ld_after_wait16(reinterpret_cast<const uint4 *>(xrow) + ch) : make_uint4(0, 0, 0, 0);
+    };
+    auto peak = [&](const uint4 &v) {
         const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) amax = max(amax, max(w[j] & 0x7fffu, (w[j] >> 16) & 0x7fffu));
-    }
+    };
+    if constexpr (NC > 0) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = max(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        for (int c = 0; c < NC; ++c) held[c] = load(c * nt + tid);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) peak(held[c]);
+    } else {
+        for (uint32_t ch = tid; ch < K / 8; ch += nt) peak(load(ch));
+    }
+    amax = __reduce_max_sync(0xffffffffu, amax);
     if (lane == 0) red[warp] = amax;
     __syncthreads();
-    if (tid == 0) {
-        uint32_t a = 0;
-        for (int i = 0; i < 8; ++i) a = max(a, red[i]);
-        int sh = 0;
-        if (a != 0 && a < 0x7f80u) {
-            const int e = (int)(a >> 7) - 127;  // floor(log2 max|x|)
-            // Bring the row maximum to [2^14 / G, 2^15 / G): every element and every
-            // group sum (at most G times the maximum) then fits f16.
-            sh = min(max(e - 14 + (int)gshift, -126), 126);
-        }
-        s_down = __int_as_float((127 - sh) << 23);
-        row_scale[m] = __int_as_float((127 + sh) << 23);
+    const uint32_t a = __reduce_max_sync(0xffffffffu, lane < nt / 32 ? red[lane] : 0u);
+    int sh = 0;
+    if (a != 0 && a < 0x7f80u) {
+        const int e = (int)(a >> 7) - 127;  // floor(log2 max|x|)
+        // Bring the row maximum to [2^14 / G, 2^15 / G): every element and every
+        // group sum (at most G times the maximum) then fits f16.
+        sh = min(max(e - 14 + (int)gshift, -126), 126);
     }
-    __syncthreads();
-    const float down = s_down;
+    const float down = __int_as_float((127 - sh) << 23);
+    if (tid == 0) row_scale[m] = __int_as_float((127 + sh) << 23);
 
-    // pass 2: convert, permute, group sums
+    // convert, permute, group sums
     const uint32_t gsize8 = (1u << gshift) / 8;  // 8-element chunks per group: 4, 8 or 16
     const uint32_t gpr = K >> gshift;
-    for (uint32_t base = 0; base < K64 / 8; base += 256) {
-        const uint32_t ch = base + tid;
-        float f[8];
-        if (ch * 8 < K) {
-            const uint4 v = dev::ld_after_wait16(reinterpret_cast<const uint4 *>(xrow) + ch);
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                f[2 * j] = __uint_as_float(w[j] << 16) * down;
-                f[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u) * down;
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) f[j] = 0.0f;
-        }
+    auto convert = [&](uint32_t ch, const uint4 &v) {
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
         __half h[8];
         float sum = 0.0f;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            h[j] = __float2half_rn(f[j]);
-            sum += __half2float(h[j]);  // the group sum is over the values the MMA will see
+        for (int j = 0; j < 4; ++j) {
+            h[2 * j] = __float2half_rn(__uint_as_float(w[j] << 16) * down);
+            h[2 * j + 1] = __float2half_rn(__uint_as_float(w[j] & 0xffff0000u) * down);
+            sum += __half2float(h[2 * j]);  // the group sum is over the values the MMA will see
+            sum += __half2float(h[2 * j + 1]);
         }
         if (ch < K64 / 8) {
             uint4 o;
@@ -147,9 +149,15 @@ __global__ void __launch_bounds__(256) x_prepare_kernel(const uint16_t *x, __hal
             q.x = pack_h2(h1, h2), q.y = pack_h2(h3, h1);
             *reinterpret_cast<uint2 *>(arow + K64 + 4 * g) = q;
         }
+    };
+    if constexpr (NC > 0) {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) convert(c * nt + tid, held[c]);
+    } else {
+        for (uint32_t base = 0; base < K64 / 8; base += nt) convert(base + tid, load(base + tid));
     }
-    // pass 3: zero the unused tail of the extra columns
-    for (uint32_t i = 4 * gpr + tid; i < K_aug - K64; i += 256) arow[K64 + i] = __float2half_rn(0.0f);
+    // zero the unused tail of the extra columns
+    for (uint32_t i = 4 * gpr + tid; i < K_aug - K64; i += nt) arow[K64 + i] = __float2half_rn(0.0f);
 }
 
 // ------------------------------------------------------------------ the GEMM ---
@@ -498,13 +506,132 @@ int pick_tile_width(uint64_t tiles_m, uint32_t n, uint32_t slots, bool pair)
     return best_bn;
 }
 
+/// How the split kernel would run a call: rows of X per tile, CTAs per tile, and an estimate of the time in ns.
+struct SplitPlan {
+    uint32_t tiles_m = 0, x_rows = 0, split = 0;
+    uint64_t cost = ~0ull;
+};
+
+/// At least this much shared memory keeps a second CTA off the SM. Each CTA holds all of its SM's TMEM: CTAs of two clusters
+/// that shared SMs crosswise would wait for each other's TMEM and never get it.
+constexpr uint32_t kSplitMinSmem = 120 * 1024;
+constexpr uint32_t kSplitMaxUsed = 6;  // 16 x 2048 rows in 6 / 8: clusters of 8 find room for 16 at most, two rounds from there
+
+/// Clusters of `split` CTAs of the split kernel that the device holds at once (a cluster lies in one GPC: 45 of three, 33 of
+/// four, 26 of five, 22 of six). The kernel's shared memory has been opted in.
+int split_clusters(TesslRuntime *rt, uint32_t split)
+{
+    const void *kernel = reinterpret_cast<const void *>(q4_prefill_gemm_split_kernel);
+    if (split == 1) return rt->sm_count;
+    int &n = rt->max_clusters[std::make_pair(kernel, split)];
+    if (n == 0) {
+        cudaLaunchConfig_t lc{};
+        lc.gridDim = dim3(split * (rt->sm_count / split)), lc.blockDim = dim3(SplitCfg::THREADS);
+        lc.dynamicSmemBytes = kSplitMinSmem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = split, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+        lc.attrs = attr, lc.numAttrs = 1;
+        const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, q4_prefill_gemm_split_kernel, &lc);
+        if (e != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            n = std::max(1, rt->sm_count / (int)split);
+        }
+    }
+    return n;
+}
+
+/// The estimates below are fits to 90 shapes (9 .. 509 rows, 512 .. 12288 x 1024 .. 17408) timed back to back, within 10 % or so.
+/// Split kernel: start and end of a tile, its part of the K blocks, and for clusters the exchange of the parts.
+Result split_plan(TesslRuntime *rt, uint32_t m, const PrefillPlan &pl, SplitPlan *out)
+{
+    TESSL_TRY(smem_opt_in(rt, reinterpret_cast<const void *>(q4_prefill_gemm_split_kernel), SplitCfg::BUDGET,
+                          "gemm_q4_mlx_tensorops: shared memory opt-in", true));
+    SplitPlan &best = *out;
+    const uint32_t tiles_m = (m + SplitCfg::MAX_X - 1) / SplitCfg::MAX_X;
+    const uint32_t x_rows = ((m + tiles_m - 1) / tiles_m + 15) & ~15u;
+    const uint64_t tiles = (uint64_t)tiles_m * ((pl.n + SplitCfg::ROWS - 1) / SplitCfg::ROWS);
+    const uint32_t blocks = pl.nkb_main + pl.nkb_extra;
+    for (uint32_t s = 1; s <= kSplitMaxUsed && blocks >= 4 * s; ++s) {
+        const uint64_t room = (uint64_t)split_clusters(rt, s), waves = (tiles + room - 1) / room;
+        const uint64_t part = (blocks + s - 1) / s;
+        const uint64_t cost = waves * ((s > 1 ? 4500 : 5200) + 8 * x_rows + part * (2000 + 3 * x_rows) / 10) +
+                              (s > 1 ? 1500 + 150 * s + 5 * s * x_rows / 2 : 0);
+        if (cost < best.cost) best = SplitPlan{tiles_m, x_rows, s, cost};
+    }
+    return ok();
+}
+
+/// CTA-pair kernel with tiles of `bn` columns: the waves of K blocks, then the last tile's stores.
+uint64_t pair_cost(uint32_t m, const PrefillPlan &pl, int bn, uint32_t clusters)
+{
+    const uint64_t tiles = (uint64_t)((m + 2 * BM - 1) / (2 * BM)) * ((pl.n + bn - 1) / bn);
+    const uint64_t waves = (tiles + clusters - 1) / clusters;
+    return 3900 + 15 * (uint64_t)bn + waves * (pl.nkb_main + pl.nkb_extra) * (1500 + 9 * (uint64_t)bn) / 10;
+}
+
+Result launch_gemm_split(TesslRuntime *rt, const TesslQ4MlxBank &bank, const TesslBuf &y, uint32_t m, OutKind out,
+                         const PrefillPlan &pl, const SplitPlan &sp, __half *a_aug, const float *row_scale)
+{
+    using C = SplitCfg;
+    EncodeTiled enc = nullptr;
+    TESSL_TRY(tensormap_encoder(rt, kWhat, &enc));
+    CUtensorMap mx, mw;
+    // X as [K block][row][64]: a unit's two tiles are one box
+    const cuuint64_t xdims[3] = {BK, m, pl.k_aug / BK}, xstrides[2] = {(cuuint64_t)pl.k_aug * 2, BK * 2};
+    const cuuint32_t xbox[3] = {BK, sp.x_rows, 2};
+    TESSL_TRY(make_map(enc, kWhat, &mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a_aug, xdims, xstrides, xbox, CU_TENSOR_MAP_SWIZZLE_128B));
+    TESSL_TRY(make_map_2d(enc, &mw, CU_TENSOR_MAP_DATA_TYPE_UINT8, bank.packed.ptr, pl.k / 2, pl.n, pl.k / 2, 64, C::ROWS,
+                          CU_TENSOR_MAP_SWIZZLE_64B));
+    // The extra units' scale words as tiles of bytes, where a row of them is a whole number of 16 bytes.
+    CUtensorMap ms = mw;
+    SplitParams p{};
+    const bool sb16 = ((uintptr_t)bank.scales_biases.ptr & 15u) == 0;
+    p.sb_tiled = sb16 && pl.groups % 4 == 0;
+    if (p.sb_tiled) {
+        TESSL_TRY(make_map_2d(enc, &ms, CU_TENSOR_MAP_DATA_TYPE_UINT8, bank.scales_biases.ptr, pl.groups * 4, pl.n, pl.groups * 4, 64,
+                              C::ROWS, CU_TENSOR_MAP_SWIZZLE_64B));
+    }
+    // A unit (two K blocks, 128 columns) has two or four words per row: one load if every row's are aligned to that.
+    p.sb_words = pl.gshift == 5 && sb16 && pl.groups % 4 == 0 ? 4 : pl.gshift == 6 && sb16 && pl.groups % 2 == 0 ? 2 : 1;
+    p.sb = static_cast<const uint32_t *>(bank.scales_biases.ptr);
+    p.row_scale = row_scale, p.y = y.ptr;
+    p.M = m, p.N = pl.n, p.gshift = pl.gshift, p.gpr = pl.groups;
+    p.nkb_main = pl.nkb_main, p.nkb_extra = pl.nkb_extra;
+    p.tiles_m = sp.tiles_m, p.x_rows = sp.x_rows, p.split = sp.split;
+    const uint32_t x_bytes = 2 * sp.x_rows * BK * 2;
+    p.su = std::min<uint32_t>(std::min<uint32_t>(C::MAX_SU, (kTmemCols - sp.x_rows) / C::UNIT_COLS), (C::BUDGET - C::FIXED) / x_bytes);
+    p.out_bf16 = out == OUT_BF16, p.status = rt->status_dev;
+    // The other CTAs' parts, at most x_rows * 512 + (split - 1) * 4096 bytes, fit over the rings: at least x_rows * 1024 + 64 KiB.
+    const size_t smem = std::max<size_t>(kSplitMinSmem, C::FIXED + (size_t)p.su * x_bytes);
+    auto kernel = q4_prefill_gemm_split_kernel;
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(sp.tiles_m * ((pl.n + C::ROWS - 1) / C::ROWS) * sp.split), lc.blockDim = dim3(C::THREADS);
+    lc.dynamicSmemBytes = smem, lc.stream = rt->stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = sp.split, attr[1].val.clusterDim.y = 1, attr[1].val.clusterDim.z = 1;
+    lc.attrs = attr, lc.numAttrs = sp.split > 1 ? 2 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&lc, kernel, mx, mw, ms, p);
+    rt->dispatch_count += 1;
+    return cuda_check(rt, e, "gemm_q4_mlx_tensorops launch");
+}
+
 /// Pre-pass and GEMM of a validated call; `scratch` holds `plan.need` bytes.
 Result prefill_launch(TesslRuntime *rt, const TesslQ4MlxBank &bank, const TesslBuf &x_bf16, const TesslBuf &y, uint32_t m,
                       OutKind out, const PrefillPlan &pl, void *scratch)
 {
     __half *a_aug = static_cast<__half *>(scratch);
     float *row_scale = reinterpret_cast<float *>(static_cast<char *>(scratch) + pl.a_bytes);
-    TESSL_TRY(launch_pdl(rt, "gemm_q4_mlx_tensorops pre-pass launch", x_prepare_kernel, dim3(m), dim3(256), 0,
+    const uint32_t chunks = pl.k64 / 8, per = (chunks + kPrepMaxThreads - 1) / kPrepMaxThreads;  // chunks per thread
+    const auto prep = per == 1 ? x_prepare_kernel<1> : per == 2 ? x_prepare_kernel<2> : x_prepare_kernel<0>;
+    const uint32_t threads = per > 2 ? kPrepMaxThreads : ((chunks + per - 1) / per + 31) & ~31u;
+    // The GEMM takes most of an SM's shared memory, and an SM changes its split of L1 and shared memory only when it is empty:
+    // with the default split the GEMM's blocks could not start on the SMs that hold rows of the pre-pass.
+    TESSL_TRY(smem_opt_in(rt, reinterpret_cast<const void *>(prep), 0, "gemm_q4_mlx_tensorops: pre-pass", true));
+    TESSL_TRY(launch_pdl(rt, "gemm_q4_mlx_tensorops pre-pass launch", prep, dim3(m), dim3(threads), 0,
                          static_cast<const uint16_t *>(x_bf16.ptr), a_aug, row_scale, pl.k, pl.k64, pl.k_aug, pl.gshift));
 
     const bool pair = rt->sm_count >= 2 && rt->prefill_force_pair != 0;
@@ -512,6 +639,17 @@ Result prefill_launch(TesslRuntime *rt, const TesslQ4MlxBank &bank, const TesslB
     const int bn = rt->prefill_force_bn
                        ? rt->prefill_force_bn
                        : pick_tile_width(tiles_m, pl.n, pair ? (uint32_t)rt->sm_count / 2 : (uint32_t)rt->sm_count, pair);
+    if (rt->prefill_force_bn == 0 && rt->prefill_force_pair < 0 && pair) {
+        SplitPlan sp;
+        TESSL_TRY(split_plan(rt, m, pl, &sp));
+        // Split kernel / pair kernel, us: 25 x 4096 x 4096 11.2 / 19.1, 509 x 2048 x 6144 23.4 / 30.4, 320 x 9216 x 2048 16.5 / 22.3,
+        // 509 x 3072 x 2048 14.4 / 15.4; and the other way: 200 x 12288 x 4096 41.2 / 29.4, 509 x 4096 x 1024 10.8 / 10.5, 420 x 3072 x
+        // 1024 10.8 / 10.2. The 3 % are for shapes where the estimates meet.
+        if (sp.cost * 100 < pair_cost(m, pl, bn, (uint32_t)rt->sm_count / 2) * 97) {
+            rt->prefill_last_bn = 64, rt->prefill_last_pair = 1;
+            return launch_gemm_split(rt, bank, y, m, out, pl, sp, a_aug, row_scale);
+        }
+    }
     rt->prefill_last_bn = bn, rt->prefill_last_pair = pair ? 1 : 0;
 
     EncodeTiled enc = nullptr;

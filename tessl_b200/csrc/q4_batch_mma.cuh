@@ -47,6 +47,7 @@ using q4k::mbar_try;
 using q4k::mbar_wait;
 using q4k::smem_u32;
 using q4k::tma_load_2d;
+using q4k::tma_load_3d;
 using q4m::lds64;
 using q4m::mma_bf16;
 
@@ -87,14 +88,6 @@ struct Params {
 struct Maps {
     CUtensorMap w[3], sb[3];
 };
-
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
-        "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
-        : "memory");
-}
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr)
 {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
