@@ -12,12 +12,14 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 LIB = HERE / "_lib" / "libtessl_b200.so"
 STEP_DRIVER = HERE / "_lib" / "tessl_step_driver"
+PY_CALL = HERE / "_lib" / "_tessl_call.so"
 SOURCES = ["capi.cu", "nn_q4.cu", "nn_q8.cu", "q4_weight.cu", "prefill_gemm.cu", "peer_gather.cu", "qwen35_norm.cu", "mlx_q4_loader.cu"]
 
 
@@ -29,10 +31,11 @@ def nvcc_path() -> str:
 
 
 def is_stale() -> bool:
-    if not LIB.exists() or not STEP_DRIVER.exists():
+    built = (LIB, STEP_DRIVER, PY_CALL)
+    if not all(b.exists() for b in built):
         return True
-    t = min(LIB.stat().st_mtime, STEP_DRIVER.stat().st_mtime)
-    deps = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + list(CSRC.glob("*.cpp"))
+    t = min(b.stat().st_mtime for b in built)
+    deps = [d for pattern in ("*.cu", "*.cuh", "*.h", "*.cpp", "*.c") for d in CSRC.glob(pattern)]
     deps.append(HERE.parent / "include" / "tessl_b200.h")
     return any(d.stat().st_mtime > t for d in deps)
 
@@ -57,6 +60,7 @@ def build(force: bool = False, verbose_ptxas: bool = False) -> Path:
     if verbose_ptxas:
         sys.stderr.write(r.stderr)
     build_step_driver(host_cxx)
+    build_py_call()
     return LIB
 
 
@@ -71,6 +75,20 @@ def build_step_driver(host_cxx=None) -> Path:
     if r.returncode != 0:
         raise RuntimeError("step driver build failed:\n$ " + " ".join(cmd) + "\n" + r.stdout + r.stderr)
     return STEP_DRIVER
+
+
+def build_py_call() -> Path:
+    """The operator calls of the Python binding (csrc/py_call.c): a CPython extension for this interpreter, linked against the
+    library beside it."""
+    cc = next((c for c in ("/usr/bin/gcc", shutil.which("gcc"), shutil.which("cc")) if c and Path(c).exists()), None)
+    if cc is None:
+        raise RuntimeError("no C compiler found")
+    cmd = [cc, "-O2", "-Wall", "-shared", "-fPIC", "-fvisibility=hidden", "-I", sysconfig.get_paths()["include"],
+           "-o", str(PY_CALL), str(CSRC / "py_call.c"), "-L", str(LIB.parent), "-ltessl_b200", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("binding build failed:\n$ " + " ".join(cmd) + "\n" + r.stdout + r.stderr)
+    return PY_CALL
 
 
 if __name__ == "__main__":

@@ -8,6 +8,8 @@ library is missing or its ABI differs, importing fails loudly.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import threading
 from pathlib import Path
 
@@ -17,6 +19,7 @@ ROW_MAJOR, INTERLEAVED4, B200_STAGED = 0, 1, 2
 GEMM_Q4_MLX_MAX_M = 8
 
 LIB_PATH = Path(__file__).resolve().parent / "_lib" / "libtessl_b200.so"
+CALL_PATH = LIB_PATH.parent / "_tessl_call.so"
 
 
 class TesslError(RuntimeError):
@@ -177,3 +180,22 @@ def call(name: str, *args) -> None:
     st = fn(*args, err, ERR_LEN)
     if st != TESSL_OK:
         raise TesslError(st, err.value.decode("utf-8", "replace"))
+
+
+_native = None
+
+
+def native():
+    """The operator calls without ctypes (csrc/py_call.c), for the library that `load` returns. Each returns True when it made
+    the call and False when it could not read an argument; a refusal is a TesslError."""
+    global _native
+    if _native is None:
+        load()
+        if not CALL_PATH.exists():
+            raise ImportError(f"{CALL_PATH} is missing: build it with `python -m tessl_b200.build`")
+        loader = importlib.machinery.ExtensionFileLoader("_tessl_call", str(CALL_PATH))
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_tessl_call", loader))
+        loader.exec_module(mod)
+        mod.set_error(TesslError)
+        _native = mod
+    return _native

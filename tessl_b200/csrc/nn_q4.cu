@@ -771,26 +771,26 @@ bool staged_domain(uint32_t cols, uint32_t group)
     return (cols / 16) / group >= 1;
 }
 
-Result check_alignment(const TesslQ4MlxBank &b, const std::string &what);
+Result check_alignment(const TesslQ4MlxBank &b, const What &what);
 
 /// The bank checks of an entry that takes either layout: the reference's for a row-major bank, size,
 /// domain and alignment of the image for a staged one.
-Result bank_validate_layout(const TesslQ4MlxBank &bank, const TesslQuantShape &shape, uint32_t layout, const std::string &what)
+Result bank_validate_layout(const TesslQ4MlxBank &bank, const TesslQuantShape &shape, uint32_t layout, const What &what)
 {
     if (layout != TESSL_Q4_B200_STAGED) return q4_bank_validate(bank, shape, what);
     TESSL_TRY(quant_shape_validate(shape, what));
     if (!staged_domain(shape.cols, shape.group_size))
         return fmt("%s: the B200 staged layout exists for rows of 1024, 2048 or 4096 columns and groups of 32, 64 or 128 "
-                   "(got %u columns, group %u)", what.c_str(), shape.cols, shape.group_size);
+                   "(got %u columns, group %u)", what.str().c_str(), shape.cols, shape.group_size);
     TESSL_TRY(require(bank.packed, nn::q4_mlx_staged_bytes(shape.rows, shape.cols, shape.group_size), 1, what + " staged image"));
     return require_aligned16(bank.packed, what + " staged image");
 }
 
-Result check_alignment(const TesslQ4MlxBank &b, const std::string &what)
+Result check_alignment(const TesslQ4MlxBank &b, const What &what)
 {
     TESSL_TRY(require_aligned16(b.packed, what + " packed"));
     if (((uintptr_t)b.scales_biases.ptr & 3u) != 0)
-        return fmt("%s scales_biases: device pointer must be 4-byte aligned", what.c_str());
+        return fmt("%s scales_biases: device pointer must be 4-byte aligned", what.str().c_str());
     return ok();
 }
 
@@ -843,15 +843,15 @@ Result gemv_q4_mlx_simd(TesslRuntime *rt, const TesslQ4MlxBank &bank, const Tess
     const bool staged = layout == TESSL_Q4_B200_STAGED;
     TESSL_TRY(refuse_layout(layout, entry, true));
     TESSL_TRY(bank_validate_layout(bank, shape, layout, entry));
-    TESSL_TRY(require(x_bf16, shape.cols, 2, std::string(entry) + " x_bf16"));
-    TESSL_TRY(require(y, shape.rows, out == OUT_BF16 ? 2 : 4, std::string(entry) + " y"));
-    if (resid) TESSL_TRY(require(*resid, shape.rows, 4, std::string(entry) + " resid"));
+    TESSL_TRY(require(x_bf16, shape.cols, 2, What(entry) + " x_bf16"));
+    TESSL_TRY(require(y, shape.rows, out == OUT_BF16 ? 2 : 4, What(entry) + " y"));
+    if (resid) TESSL_TRY(require(*resid, shape.rows, 4, What(entry) + " resid"));
     if (shape.rows == 0) return ok();
     const Named writes[] = {{"y", &y}};
     const Named reads[] = {{"packed", &bank.packed}, {"scales_biases", &bank.scales_biases}, {"x_bf16", &x_bf16}};
     TESSL_TRY(require_disjoint_writes(entry, writes, 1, reads, 3));
     if (!staged) TESSL_TRY(check_alignment(bank, entry));
-    TESSL_TRY(require_aligned16(x_bf16, std::string(entry) + " x_bf16"));
+    TESSL_TRY(require_aligned16(x_bf16, What(entry) + " x_bf16"));
     if (shape.cols == 0) {
         // No columns: every sum is empty. The kernel's loop never runs and the
         // epilogue stores 0 (+ resid), as the reference's does.
@@ -874,13 +874,13 @@ Result gemv_q4_mlx_gate_up(TesslRuntime *rt, const char *entry, const char *what
 {
     const bool staged = layout == TESSL_Q4_B200_STAGED;
     TESSL_TRY(refuse_layout(layout, entry, true));
-    TESSL_TRY(bank_validate_layout(gate, shape, layout, std::string(entry) + " gate"));
-    TESSL_TRY(bank_validate_layout(up, shape, layout, std::string(entry) + " up"));
-    TESSL_TRY(require(x, shape.cols, 2, std::string(entry) + " x"));
+    TESSL_TRY(bank_validate_layout(gate, shape, layout, What(entry) + " gate"));
+    TESSL_TRY(bank_validate_layout(up, shape, layout, What(entry) + " up"));
+    TESSL_TRY(require(x, shape.cols, 2, What(entry) + " x"));
     if (mid_as_bf16) {
-        TESSL_TRY(require(mid, shape.rows, 2, std::string(entry) + " mid (bf16)"));
+        TESSL_TRY(require(mid, shape.rows, 2, What(entry) + " mid (bf16)"));
     } else {
-        TESSL_TRY(require(mid, shape.rows, 4, std::string(entry) + " mid"));
+        TESSL_TRY(require(mid, shape.rows, 4, What(entry) + " mid"));
     }
     if (shape.rows == 0) return ok();
     const Named writes[] = {{"mid", &mid}};
@@ -891,10 +891,10 @@ Result gemv_q4_mlx_gate_up(TesslRuntime *rt, const char *entry, const char *what
                            {"x", &x}};
     TESSL_TRY(require_disjoint_writes(what, writes, 1, reads, 5));
     if (!staged) {
-        TESSL_TRY(check_alignment(gate, std::string(entry) + " gate"));
-        TESSL_TRY(check_alignment(up, std::string(entry) + " up"));
+        TESSL_TRY(check_alignment(gate, What(entry) + " gate"));
+        TESSL_TRY(check_alignment(up, What(entry) + " up"));
     }
-    TESSL_TRY(require_aligned16(x, std::string(entry) + " x"));
+    TESSL_TRY(require_aligned16(x, What(entry) + " x"));
     Q4GemvParams p{};
     p.staged = staged;
     p.seg[0] = make_seg(gate, &up, mid, nullptr, shape.rows);
@@ -927,12 +927,12 @@ Result gemv_q4_mlx_simd_sharded(TesslRuntime *rt, const TesslQ4MlxBank &bank, co
     TESSL_TRY(sharded_out(gather, entry, (uint64_t)shape.rows * (y_as_bf16 ? 2 : 4), &y));
     if (shape.rows == 0) return fmt("%s: a rank with no rows takes part through tessl_peer_gather", entry);
     TESSL_TRY(q4_bank_validate(bank, shape, entry));
-    TESSL_TRY(require(x_bf16, shape.cols, 2, std::string(entry) + " x_bf16"));
+    TESSL_TRY(require(x_bf16, shape.cols, 2, What(entry) + " x_bf16"));
     const Named writes[] = {{"gather slot", &y}};
     const Named reads[] = {{"packed", &bank.packed}, {"scales_biases", &bank.scales_biases}, {"x_bf16", &x_bf16}};
     TESSL_TRY(require_disjoint_writes(entry, writes, 1, reads, 3));
     TESSL_TRY(check_alignment(bank, entry));
-    TESSL_TRY(require_aligned16(x_bf16, std::string(entry) + " x_bf16"));
+    TESSL_TRY(require_aligned16(x_bf16, What(entry) + " x_bf16"));
     Q4GemvParams p{};
     p.seg[0] = make_seg(bank, nullptr, y, nullptr, shape.rows);
     p.nseg = 1;
@@ -955,9 +955,9 @@ Result gemv_q4_mlx_simd_gathered(TesslRuntime *rt, const TesslQ4MlxBank &bank, c
     x.ptr = gather.buffers[gather.rank];
     x.nbytes = (uint64_t)gather.world * gather.bytes_per_rank;
     TESSL_TRY(q4_bank_validate(bank, shape, entry));
-    TESSL_TRY(require(x, shape.cols, 2, std::string(entry) + " gathered x"));
-    TESSL_TRY(require(y, shape.rows, out == OUT_BF16 ? 2 : 4, std::string(entry) + " y"));
-    if (resid) TESSL_TRY(require(*resid, shape.rows, 4, std::string(entry) + " resid"));
+    TESSL_TRY(require(x, shape.cols, 2, What(entry) + " gathered x"));
+    TESSL_TRY(require(y, shape.rows, out == OUT_BF16 ? 2 : 4, What(entry) + " y"));
+    if (resid) TESSL_TRY(require(*resid, shape.rows, 4, What(entry) + " resid"));
     if (shape.rows == 0) return ok();
     const Named writes[] = {{"y", &y}};
     const Named reads[] = {{"packed", &bank.packed}, {"scales_biases", &bank.scales_biases}, {"gathered x", &x}};
@@ -983,9 +983,9 @@ Result gemv_q4_mlx_gate_up_silu_sharded(TesslRuntime *rt, const TesslQ4MlxBank &
     TesslBuf mid{};
     TESSL_TRY(sharded_out(gather, entry, (uint64_t)shape.rows * (mid_as_bf16 ? 2 : 4), &mid));
     if (shape.rows == 0) return fmt("%s: a rank with no rows takes part through tessl_peer_gather", entry);
-    TESSL_TRY(q4_bank_validate(gate, shape, std::string(entry) + " gate"));
-    TESSL_TRY(q4_bank_validate(up, shape, std::string(entry) + " up"));
-    TESSL_TRY(require(x, shape.cols, 2, std::string(entry) + " x"));
+    TESSL_TRY(q4_bank_validate(gate, shape, What(entry) + " gate"));
+    TESSL_TRY(q4_bank_validate(up, shape, What(entry) + " up"));
+    TESSL_TRY(require(x, shape.cols, 2, What(entry) + " x"));
     const Named writes[] = {{"gather slot", &mid}};
     const Named reads[] = {{"gate_packed", &gate.packed},
                            {"gate_scales_biases", &gate.scales_biases},
@@ -993,9 +993,9 @@ Result gemv_q4_mlx_gate_up_silu_sharded(TesslRuntime *rt, const TesslQ4MlxBank &
                            {"up_scales_biases", &up.scales_biases},
                            {"x", &x}};
     TESSL_TRY(require_disjoint_writes(entry, writes, 1, reads, 5));
-    TESSL_TRY(check_alignment(gate, std::string(entry) + " gate"));
-    TESSL_TRY(check_alignment(up, std::string(entry) + " up"));
-    TESSL_TRY(require_aligned16(x, std::string(entry) + " x"));
+    TESSL_TRY(check_alignment(gate, What(entry) + " gate"));
+    TESSL_TRY(check_alignment(up, What(entry) + " up"));
+    TESSL_TRY(require_aligned16(x, What(entry) + " x"));
     Q4GemvParams p{};
     p.seg[0] = make_seg(gate, &up, mid, nullptr, shape.rows);
     p.nseg = 1;
@@ -1014,11 +1014,11 @@ Result gemv_q4_mlx_kv(TesslRuntime *rt, const TesslQ4MlxBank &k, const TesslQ4Ml
 {
     const char *entry = "gemv_q4_mlx_simd_kv";
     TESSL_TRY(refuse_layout(layout, entry));
-    TESSL_TRY(q4_bank_validate(k, shape, std::string(entry) + " k"));
-    TESSL_TRY(q4_bank_validate(v, shape, std::string(entry) + " v"));
-    TESSL_TRY(require(x_bf16, shape.cols, 2, std::string(entry) + " x_bf16"));
-    TESSL_TRY(require(k_out, shape.rows, 4, std::string(entry) + " k_out"));
-    TESSL_TRY(require(v_out, shape.rows, 4, std::string(entry) + " v_out"));
+    TESSL_TRY(q4_bank_validate(k, shape, What(entry) + " k"));
+    TESSL_TRY(q4_bank_validate(v, shape, What(entry) + " v"));
+    TESSL_TRY(require(x_bf16, shape.cols, 2, What(entry) + " x_bf16"));
+    TESSL_TRY(require(k_out, shape.rows, 4, What(entry) + " k_out"));
+    TESSL_TRY(require(v_out, shape.rows, 4, What(entry) + " v_out"));
     if (shape.rows == 0) return ok();
     const Named writes[] = {{"k_out", &k_out}, {"v_out", &v_out}};
     const Named reads[] = {{"k_packed", &k.packed},
@@ -1027,9 +1027,9 @@ Result gemv_q4_mlx_kv(TesslRuntime *rt, const TesslQ4MlxBank &k, const TesslQ4Ml
                            {"v_scales_biases", &v.scales_biases},
                            {"x_bf16", &x_bf16}};
     TESSL_TRY(require_disjoint_writes("gemv_q4_mlx_kv", writes, 2, reads, 5));
-    TESSL_TRY(check_alignment(k, std::string(entry) + " k"));
-    TESSL_TRY(check_alignment(v, std::string(entry) + " v"));
-    TESSL_TRY(require_aligned16(x_bf16, std::string(entry) + " x_bf16"));
+    TESSL_TRY(check_alignment(k, What(entry) + " k"));
+    TESSL_TRY(check_alignment(v, What(entry) + " v"));
+    TESSL_TRY(require_aligned16(x_bf16, What(entry) + " x_bf16"));
     Q4GemvParams p{};
     p.seg[0] = make_seg(k, nullptr, k_out, nullptr, shape.rows);
     p.seg[1] = make_seg(v, nullptr, v_out, nullptr, shape.rows);
@@ -1048,13 +1048,13 @@ Result gemv_q4_mlx_qkv(TesslRuntime *rt, const TesslQ4MlxBank &q, const TesslQ4M
     const char *entry = "gemv_q4_mlx_simd_qkv";
     TESSL_TRY(refuse_layout(layout, entry));
     const TesslQuantShape q_shape{rows_q, cols, group_size}, kv_shape{rows_kv, cols, group_size};
-    TESSL_TRY(q4_bank_validate(q, q_shape, std::string(entry) + " q"));
-    TESSL_TRY(q4_bank_validate(k, kv_shape, std::string(entry) + " k"));
-    TESSL_TRY(q4_bank_validate(v, kv_shape, std::string(entry) + " v"));
-    TESSL_TRY(require(x_bf16, cols, 2, std::string(entry) + " x_bf16"));
-    TESSL_TRY(require(out.q_out, rows_q, 4, std::string(entry) + " q_out"));
-    TESSL_TRY(require(out.k_out, rows_kv, 4, std::string(entry) + " k_out"));
-    TESSL_TRY(require(out.v_out, rows_kv, 4, std::string(entry) + " v_out"));
+    TESSL_TRY(q4_bank_validate(q, q_shape, What(entry) + " q"));
+    TESSL_TRY(q4_bank_validate(k, kv_shape, What(entry) + " k"));
+    TESSL_TRY(q4_bank_validate(v, kv_shape, What(entry) + " v"));
+    TESSL_TRY(require(x_bf16, cols, 2, What(entry) + " x_bf16"));
+    TESSL_TRY(require(out.q_out, rows_q, 4, What(entry) + " q_out"));
+    TESSL_TRY(require(out.k_out, rows_kv, 4, What(entry) + " k_out"));
+    TESSL_TRY(require(out.v_out, rows_kv, 4, What(entry) + " v_out"));
     if (rows_q == 0 && rows_kv == 0) return ok();
     // Only the banks that produce output take part in the aliasing check.
     Named writes[3];
@@ -1075,16 +1075,16 @@ Result gemv_q4_mlx_qkv(TesslRuntime *rt, const TesslQ4MlxBank &q, const TesslQ4M
     }
     reads[nr++] = {"x_bf16", &x_bf16};
     TESSL_TRY(require_disjoint_writes(entry, writes, nw, reads, nr));
-    TESSL_TRY(require_aligned16(x_bf16, std::string(entry) + " x_bf16"));
+    TESSL_TRY(require_aligned16(x_bf16, What(entry) + " x_bf16"));
     Q4GemvParams p{};
     p.nseg = 0;
     if (rows_q != 0) {
-        TESSL_TRY(check_alignment(q, std::string(entry) + " q"));
+        TESSL_TRY(check_alignment(q, What(entry) + " q"));
         p.seg[p.nseg++] = make_seg(q, nullptr, out.q_out, nullptr, rows_q);
     }
     if (rows_kv != 0) {
-        TESSL_TRY(check_alignment(k, std::string(entry) + " k"));
-        TESSL_TRY(check_alignment(v, std::string(entry) + " v"));
+        TESSL_TRY(check_alignment(k, What(entry) + " k"));
+        TESSL_TRY(check_alignment(v, What(entry) + " v"));
         p.seg[p.nseg++] = make_seg(k, nullptr, out.k_out, nullptr, rows_kv);
         p.seg[p.nseg++] = make_seg(v, nullptr, out.v_out, nullptr, rows_kv);
     }
@@ -1148,15 +1148,15 @@ Result gemm_q4_mlx(TesslRuntime *rt, const TesslQ4MlxBank &bank, const TesslBuf 
     }
     TESSL_TRY(q4_bank_validate(bank, shape, entry));
     const uint64_t out_elems = elems(m, shape.rows);
-    TESSL_TRY(require(x_bf16, elems(m, shape.cols), 2, std::string(entry) + " x_bf16"));
-    TESSL_TRY(require(y, out_elems, out == OUT_BF16 ? 2 : 4, std::string(entry) + " y"));
-    if (resid) TESSL_TRY(require(*resid, out_elems, 4, std::string(entry) + " resid"));
+    TESSL_TRY(require(x_bf16, elems(m, shape.cols), 2, What(entry) + " x_bf16"));
+    TESSL_TRY(require(y, out_elems, out == OUT_BF16 ? 2 : 4, What(entry) + " y"));
+    if (resid) TESSL_TRY(require(*resid, out_elems, 4, What(entry) + " resid"));
     if (shape.rows == 0) return ok();
     const Named writes[] = {{"y", &y}};
     const Named reads[] = {{"packed", &bank.packed}, {"scales_biases", &bank.scales_biases}, {"x_bf16", &x_bf16}};
     TESSL_TRY(require_disjoint_writes("gemm_q4_mlx", writes, 1, reads, 3));
     TESSL_TRY(check_alignment(bank, entry));
-    TESSL_TRY(require_aligned16(x_bf16, std::string(entry) + " x_bf16"));
+    TESSL_TRY(require_aligned16(x_bf16, What(entry) + " x_bf16"));
     Q4GemvParams p{};
     p.seg[0] = make_seg(bank, nullptr, y, resid, shape.rows);
     p.nseg = 1;
@@ -1175,14 +1175,14 @@ Result embed_lookup_q4_mlx(TesslRuntime *rt, const TesslQ4MlxBank &bank, const T
     const TesslQuantShape shape{vocab, hidden, group_size};
     TESSL_TRY(q4_bank_validate(bank, shape, what));
     const uint64_t total = elems(n_tokens, hidden);
-    TESSL_TRY(require(token_ids, n_tokens, 4, std::string(what) + " token_ids"));
-    TESSL_TRY(require(out, total, 4, std::string(what) + " out"));
+    TESSL_TRY(require(token_ids, n_tokens, 4, What(what) + " token_ids"));
+    TESSL_TRY(require(out, total, 4, What(what) + " out"));
     const Named writes[] = {{"out", &out}};
     const Named reads[] = {{"packed", &bank.packed}, {"scales_biases", &bank.scales_biases}, {"token_ids", &token_ids}};
     TESSL_TRY(require_disjoint_writes(what, writes, 1, reads, 3));
     if (total == 0) return ok();
     TESSL_TRY(check_alignment(bank, what));
-    TESSL_TRY(require_aligned16(out, std::string(what) + " out"));
+    TESSL_TRY(require_aligned16(out, What(what) + " out"));
     if (((uintptr_t)token_ids.ptr & 3u) != 0) return fmt("%s token_ids: device pointer must be 4-byte aligned", what);
     const uint64_t total32 = total / 32;  // hidden is a multiple of the group size, itself a multiple of 32
     return launch_pdl(rt, "embed_lookup_q4_mlx launch", embed_lookup_q4_mlx_kernel, dim3((unsigned)((total32 + 127) / 128)), dim3(128), 0,
@@ -1205,14 +1205,14 @@ Result q4_mlx_repack_staged(TesslRuntime *rt, const TesslQ4MlxBank &bank, const 
         return fmt("%s: the B200 staged layout exists for rows of 1024, 2048 or 4096 columns and groups of 32, 64 or 128 "
                    "(got %u columns, group %u)", entry, shape.cols, shape.group_size);
     const uint64_t nbytes = q4_mlx_staged_bytes(shape.rows, shape.cols, shape.group_size);
-    TESSL_TRY(require(out, nbytes, 1, std::string(entry) + " out"));
+    TESSL_TRY(require(out, nbytes, 1, What(entry) + " out"));
     if (shape.rows == 0) return ok();
     const Named writes[] = {{"out", &out}};
     const Named reads[] = {{"packed", &bank.packed}, {"scales_biases", &bank.scales_biases}};
     TESSL_TRY(require_disjoint_writes(entry, writes, 1, reads, 2));
-    TESSL_TRY(require_aligned16(bank.packed, std::string(entry) + " packed"));
-    TESSL_TRY(require_aligned16(bank.scales_biases, std::string(entry) + " scales_biases"));
-    TESSL_TRY(require_aligned16(out, std::string(entry) + " out"));
+    TESSL_TRY(require_aligned16(bank.packed, What(entry) + " packed"));
+    TESSL_TRY(require_aligned16(bank.scales_biases, What(entry) + " scales_biases"));
+    TESSL_TRY(require_aligned16(out, What(entry) + " out"));
     const uint64_t n16 = nbytes / 16;
     q4_repack_staged_kernel<<<(unsigned)((n16 + 255) / 256), 256, 0, rt->stream>>>(
         static_cast<const uint4 *>(bank.packed.ptr), static_cast<const uint4 *>(bank.scales_biases.ptr),

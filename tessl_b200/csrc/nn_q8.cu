@@ -291,17 +291,17 @@ Result gemm_q8_mlx(TesslRuntime *rt, const TesslBuf &codes, const TesslBuf &sb, 
         return fmt("%s: group_size %u is outside the MLX kernel domain {32, 64, 128, 256, 512}", entry,
                    shape.group_size);
     }
-    TESSL_TRY(require(codes, elems(shape.rows, shape.cols), 1, std::string(entry) + " codes"));
+    TESSL_TRY(require(codes, elems(shape.rows, shape.cols), 1, What(entry) + " codes"));
     TESSL_TRY(require(sb, elems(shape.rows, shape.cols / shape.group_size), 4,
-                      std::string(entry) + " scales_biases (bfloat2 per group)"));
-    TESSL_TRY(require(x_bf16, elems(m, shape.cols), 2, std::string(entry) + " x_bf16"));
-    TESSL_TRY(require(y, elems(m, shape.rows), out == OUT_BF16 ? 2 : 4, std::string(entry) + " y"));
+                      What(entry) + " scales_biases (bfloat2 per group)"));
+    TESSL_TRY(require(x_bf16, elems(m, shape.cols), 2, What(entry) + " x_bf16"));
+    TESSL_TRY(require(y, elems(m, shape.rows), out == OUT_BF16 ? 2 : 4, What(entry) + " y"));
     if (shape.rows == 0) return ok();
     const Named writes[] = {{"y", &y}};
     const Named reads[] = {{"codes", &codes}, {"scales_biases", &sb}, {"x_bf16", &x_bf16}};
     TESSL_TRY(require_disjoint_writes(entry, writes, 1, reads, 3));
-    TESSL_TRY(require_aligned16(codes, std::string(entry) + " codes"));
-    TESSL_TRY(require_aligned16(x_bf16, std::string(entry) + " x_bf16"));
+    TESSL_TRY(require_aligned16(codes, What(entry) + " codes"));
+    TESSL_TRY(require_aligned16(x_bf16, What(entry) + " x_bf16"));
     {
         // rows of 512 .. 4096 codes in groups of 32 or 64: the tensor-core GEMV kernel (q4_gemv_mma.cuh)
         bool handled = false;

@@ -458,16 +458,16 @@ Result prefill_validate(const TesslQ4MlxBank &bank, const TesslBuf &x_bf16, cons
     TESSL_TRY(require_i32_extent(elems(m, n), "gemm_q4_mlx_tensorops y (m * rows)"));
     TESSL_TRY(require_i32_extent(elems(n, groups), "gemm_q4_mlx_tensorops scale/bias pairs (rows * groups)"));
     TESSL_TRY(q4_bank_validate(bank, shape, what));
-    TESSL_TRY(require(x_bf16, elems(m, k), 2, std::string(what) + " x_bf16"));
-    TESSL_TRY(require(y, elems(m, n), out == OUT_BF16 ? 2 : 4, std::string(what) + " y"));
+    TESSL_TRY(require(x_bf16, elems(m, k), 2, What(what) + " x_bf16"));
+    TESSL_TRY(require(y, elems(m, n), out == OUT_BF16 ? 2 : 4, What(what) + " y"));
     const Named writes[] = {{"y", &y}};
     const Named reads[] = {{"packed", &bank.packed}, {"scales_biases", &bank.scales_biases}, {"x_bf16", &x_bf16}};
     TESSL_TRY(require_disjoint_writes(what, writes, 1, reads, 3));
     *empty = m == 0 || n == 0;
     if (*empty) return ok();
-    TESSL_TRY(require_aligned16(bank.packed, std::string(what) + " packed"));
-    TESSL_TRY(require_aligned16(x_bf16, std::string(what) + " x_bf16"));
-    TESSL_TRY(require_aligned16(y, std::string(what) + " y"));
+    TESSL_TRY(require_aligned16(bank.packed, What(what) + " packed"));
+    TESSL_TRY(require_aligned16(x_bf16, What(what) + " x_bf16"));
+    TESSL_TRY(require_aligned16(y, What(what) + " y"));
     if (((uintptr_t)bank.scales_biases.ptr & 3u) != 0)
         return fmt("%s scales_biases: device pointer must be 4-byte aligned", what);
 

@@ -148,17 +148,40 @@ inline Result scratch_reserve(TesslRuntime *rt, size_t bytes, void **out)
 
 // ------------------------------------------------------------ validation ---
 
+/// What a refusal names, in up to four pieces that are put together only when one is written: composed up front, the names
+/// of a call that succeeds were most of its validation (~10 strings on the heap per GEMV).
+class What {
+public:
+    What(const char *s) : part_{s}, n_(1) {}
+    What operator+(const char *s) const
+    {
+        What w = *this;
+        if (w.n_ < 4) w.part_[w.n_++] = s;
+        return w;
+    }
+    std::string str() const
+    {
+        std::string s;
+        for (int i = 0; i < n_; ++i) s += part_[i];
+        return s;
+    }
+
+private:
+    const char *part_[4];
+    int n_;
+};
+
 inline uint64_t elems(uint32_t a, uint32_t b) { return uint64_t(a) * uint64_t(b); }
 
 /// `nn::require::<T>` (src/nn.rs:126-143): capacity in elements of `elem` bytes.
-inline Result require(const TesslBuf &buf, uint64_t need, size_t elem, const std::string &what)
+inline Result require(const TesslBuf &buf, uint64_t need, size_t elem, const What &what)
 {
     const uint64_t have = buf.nbytes / elem;
     if (have < need) {
-        return fmt("%s: buffer holds %llu elements, kernel reads/writes %llu", what.c_str(),
+        return fmt("%s: buffer holds %llu elements, kernel reads/writes %llu", what.str().c_str(),
                    (unsigned long long)have, (unsigned long long)need);
     }
-    if (need > 0 && buf.ptr == nullptr) return fmt("%s: null device pointer", what.c_str());
+    if (need > 0 && buf.ptr == nullptr) return fmt("%s: null device pointer", what.str().c_str());
     return ok();
 }
 
@@ -193,19 +216,19 @@ inline Result require_disjoint_writes(const char *entry, const Named *writes, in
 }
 
 /// `QuantShape::validate` (src/nn.rs:3254-3267).
-inline Result quant_shape_validate(const TesslQuantShape &s, const std::string &what)
+inline Result quant_shape_validate(const TesslQuantShape &s, const What &what)
 {
-    if (s.group_size == 0) return fmt("%s: group_size must be non-zero", what.c_str());
+    if (s.group_size == 0) return fmt("%s: group_size must be non-zero", what.str().c_str());
     if (s.cols % s.group_size != 0) {
         return fmt("%s: cols %u is not a multiple of group_size %u; the kernels compute `cols / group_size` "
                    "with integer division and would silently drop the ragged tail group",
-                   what.c_str(), s.cols, s.group_size);
+                   what.str().c_str(), s.cols, s.group_size);
     }
     return ok();
 }
 
 /// `Q4MlxBank::validate` for a row-major bank (src/nn.rs:3348-3385).
-inline Result q4_bank_validate(const TesslQ4MlxBank &bank, const TesslQuantShape &s, const std::string &what)
+inline Result q4_bank_validate(const TesslQ4MlxBank &bank, const TesslQuantShape &s, const What &what)
 {
     Result r = quant_shape_validate(s, what);
     if (!r.empty()) return r;
@@ -213,7 +236,7 @@ inline Result q4_bank_validate(const TesslQ4MlxBank &bank, const TesslQuantShape
         return fmt("%s: group_size %u is outside the MLX kernel domain {32, 64, 128, 256, 512}; the row kernels "
                    "peel each group through 16-byte loads and the simdgroup kernels stride their scale pointer "
                    "by 512 / group_size",
-                   what.c_str(), s.group_size);
+                   what.str().c_str(), s.group_size);
     }
     const uint64_t groups = elems(s.rows, s.cols / s.group_size);
     const uint64_t weights = elems(s.rows, s.cols);
@@ -224,9 +247,9 @@ inline Result q4_bank_validate(const TesslQ4MlxBank &bank, const TesslQuantShape
 
 /// The kernels read packed rows and activations with 16-byte loads; CUDA
 /// allocations are 256-byte aligned, so only a caller-made sub-view can trip this.
-inline Result require_aligned16(const TesslBuf &b, const std::string &what)
+inline Result require_aligned16(const TesslBuf &b, const What &what)
 {
-    if (((uintptr_t)b.ptr & 15u) != 0) return fmt("%s: device pointer must be 16-byte aligned", what.c_str());
+    if (((uintptr_t)b.ptr & 15u) != 0) return fmt("%s: device pointer must be 16-byte aligned", what.str().c_str());
     return ok();
 }
 

@@ -4,7 +4,8 @@ Names, argument order and refusals follow `src/nn.rs` and `src/qwen35_q4.rs`
 of the reference project (`nn::gemv_q4_mlx_simd`, `nn::gemm_q4_mlx`,
 `nn::gemm_q4_mlx_tensorops`, `nn::gemv_q8`, `Q4Weight::matmul`, ...); every
 function forwards to the C ABI of `libtessl_b200.so`, where validation and the
-CUDA launches live. A refusal surfaces as `TesslError` carrying the library's
+CUDA launches live: the operators through the native call module (csrc/py_call.c), which
+hands arguments that it cannot read back to ctypes. A refusal surfaces as `TesslError` carrying the library's
 message. Nothing here computes: without the CUDA library the import fails.
 """
 from __future__ import annotations
@@ -208,6 +209,18 @@ def _opt(buf: Optional[GpuBuffer]):
     return None if buf is None else C.byref(buf.c())
 
 
+class _Native:
+    """The native calls, bound on first use: importing this module does not need the library."""
+
+    def __getattr__(self, name):
+        fn = getattr(capi.native(), name)
+        setattr(self, name, fn)
+        return fn
+
+
+_native = _Native()
+
+
 def simd_gemv_threadgroups(rows: int) -> int:
     """`nn::simd_gemv_threadgroups` (src/nn.rs:3699-3701)."""
     return capi.load().tessl_simd_gemv_threadgroups(rows)
@@ -216,6 +229,8 @@ def simd_gemv_threadgroups(rows: int) -> int:
 def gemv_q4_mlx_simd(rt: Runtime, bank: Q4MlxBank, x_bf16: GpuBuffer, y: GpuBuffer, shape: QuantShape,
                      layout: int = ROW_MAJOR, resid: Optional[GpuBuffer] = None, *, y_as_bf16: bool = False) -> None:
     """`nn::gemv_q4_mlx_simd` (src/nn.rs:3982-4074). `y_as_bf16` selects the bf16-output twin."""
+    if _native.gemv_q4_mlx_simd(rt, bank, x_bf16, y, shape, layout, resid, y_as_bf16):
+        return
     name = "tessl_gemv_q4_mlx_simd_bf16" if y_as_bf16 else "tessl_gemv_q4_mlx_simd"
     capi.call(name, rt.handle, bank.c(), x_bf16.c(), y.c(), shape.c(), layout, _opt(resid))
 
@@ -225,6 +240,8 @@ def gemv_q4_mlx_gate_up_silu(rt: Runtime, gate: Q4MlxBank, up: Q4MlxBank, x: Gpu
     """`nn::gemv_q4_mlx_gate_up_silu` (src/nn.rs:4165-4194); `layout` other than row-major goes through the
     library's own entry with a layout argument."""
     if layout == ROW_MAJOR:
+        if _native.gemv_q4_mlx_gate_up_silu(rt, gate, up, x, mid, shape, mid_as_bf16):
+            return
         capi.call("tessl_gemv_q4_mlx_gate_up_silu", rt.handle, gate.c(), up.c(), x.c(), mid.c(), shape.c(),
                   int(mid_as_bf16))
     else:
@@ -258,24 +275,32 @@ def gemv_q4_mlx_gate_up_gelu(rt: Runtime, gate: Q4MlxBank, up: Q4MlxBank, x: Gpu
 def gemv_q4_mlx_kv(rt: Runtime, k: Q4MlxBank, v: Q4MlxBank, x_bf16: GpuBuffer, k_out: GpuBuffer, v_out: GpuBuffer,
                    shape: QuantShape, layout: int = ROW_MAJOR) -> None:
     """`nn::gemv_q4_mlx_kv` (src/nn.rs:4279-4351)."""
+    if _native.gemv_q4_mlx_kv(rt, k, v, x_bf16, k_out, v_out, shape, layout):
+        return
     capi.call("tessl_gemv_q4_mlx_kv", rt.handle, k.c(), v.c(), x_bf16.c(), k_out.c(), v_out.c(), shape.c(), layout)
 
 
 def gemv_q4_mlx_qkv(rt: Runtime, q: Q4MlxBank, k: Q4MlxBank, v: Q4MlxBank, x_bf16: GpuBuffer, out: QkvOutputs,
                     rows_q: int, rows_kv: int, cols: int, group_size: int, layout: int = ROW_MAJOR) -> None:
     """`nn::gemv_q4_mlx_qkv` (src/nn.rs:4366-4515)."""
+    if _native.gemv_q4_mlx_qkv(rt, q, k, v, x_bf16, out, rows_q, rows_kv, cols, group_size, layout):
+        return
     capi.call("tessl_gemv_q4_mlx_qkv", rt.handle, q.c(), k.c(), v.c(), x_bf16.c(), out.c(), rows_q, rows_kv, cols,
               group_size, layout)
 
 
 def swiglu(rt: Runtime, gate: GpuBuffer, up: GpuBuffer, out: GpuBuffer, n: int, out_as_bf16: bool) -> None:
     """`qwen35::swiglu` as the unfused gate/up path uses it (src/qwen35_model.rs:1938-1957)."""
+    if _native.swiglu(rt, gate, up, out, n, out_as_bf16):
+        return
     capi.call("tessl_swiglu", rt.handle, gate.c(), up.c(), out.c(), n, int(out_as_bf16))
 
 
 def gemm_q4_mlx(rt: Runtime, bank: Q4MlxBank, x_bf16: GpuBuffer, y: GpuBuffer, shape: QuantShape, m: int,
                 layout: int = ROW_MAJOR, resid: Optional[GpuBuffer] = None, *, y_as_bf16: bool = False) -> None:
     """`nn::gemm_q4_mlx` (src/nn.rs:4535-4619): m <= 8."""
+    if _native.gemm_q4_mlx(rt, bank, x_bf16, y, shape, m, layout, resid, y_as_bf16):
+        return
     name = "tessl_gemm_q4_mlx_bf16" if y_as_bf16 else "tessl_gemm_q4_mlx"
     capi.call(name, rt.handle, bank.c(), x_bf16.c(), y.c(), shape.c(), m, layout, _opt(resid))
 
@@ -288,6 +313,8 @@ def gemm_q4_mlx_tensorops_max_k(m: int, n: int, group_size: int) -> int:
 def gemm_q4_mlx_tensorops(rt: Runtime, bank: Q4MlxBank, x_bf16: GpuBuffer, y: GpuBuffer, shape: QuantShape, m: int,
                           *, y_as_bf16: bool = False) -> None:
     """`nn::gemm_q4_mlx_tensorops` (src/nn.rs:4683-4757): the prefill GEMM."""
+    if _native.gemm_q4_mlx_tensorops(rt, bank, x_bf16, y, shape, m, y_as_bf16):
+        return
     name = "tessl_gemm_q4_mlx_tensorops_bf16" if y_as_bf16 else "tessl_gemm_q4_mlx_tensorops"
     capi.call(name, rt.handle, bank.c(), x_bf16.c(), y.c(), shape.c(), m)
 
@@ -303,12 +330,16 @@ def gemm_q4_mlx_tensorops_noalloc(rt: Runtime, bank: Q4MlxBank, x_bf16: GpuBuffe
 def gemv_q8(rt: Runtime, packed: GpuBuffer, scales: GpuBuffer, zeros: GpuBuffer, x: GpuBuffer, y: GpuBuffer,
             rows: int, cols: int, group_size: int) -> None:
     """`nn::gemv_q8` (src/nn.rs:716-795)."""
+    if _native.gemv_q8(rt, packed, scales, zeros, x, y, rows, cols, group_size):
+        return
     capi.call("tessl_gemv_q8", rt.handle, packed.c(), scales.c(), zeros.c(), x.c(), y.c(), rows, cols, group_size)
 
 
 def gemm_q8_mlx(rt: Runtime, codes: GpuBuffer, scales_biases: GpuBuffer, x_bf16: GpuBuffer, y: GpuBuffer,
                 shape: QuantShape, m: int, y_as_bf16: bool = False) -> None:
     """MLX-layout 8-bit GEMV/GEMM for m <= 8 (no counterpart in the reference)."""
+    if _native.gemm_q8_mlx(rt, codes, scales_biases, x_bf16, y, shape, m, y_as_bf16):
+        return
     capi.call("tessl_gemm_q8_mlx", rt.handle, codes.c(), scales_biases.c(), x_bf16.c(), y.c(), shape.c(), m,
               int(y_as_bf16))
 
@@ -316,6 +347,8 @@ def gemm_q8_mlx(rt: Runtime, codes: GpuBuffer, scales_biases: GpuBuffer, x_bf16:
 def embed_lookup_q4_mlx(rt: Runtime, bank: Q4MlxBank, token_ids: GpuBuffer, out: GpuBuffer, vocab: int, hidden: int,
                         group_size: int, n_tokens: int) -> None:
     """`nn::embed_lookup_q4_mlx` (src/nn.rs:3592-3658): gather dequantized rows; ids >= vocab give zeros."""
+    if _native.embed_lookup_q4_mlx(rt, bank, token_ids, out, vocab, hidden, group_size, n_tokens):
+        return
     capi.call("tessl_embed_lookup_q4_mlx", rt.handle, bank.c(), token_ids.c(), out.c(), vocab, hidden, group_size,
               n_tokens)
 
@@ -323,17 +356,23 @@ def embed_lookup_q4_mlx(rt: Runtime, bank: Q4MlxBank, token_ids: GpuBuffer, out:
 def qwen35_rms_norm(rt: Runtime, x: GpuBuffer, w: GpuBuffer, out: GpuBuffer, out_as_bf16: bool, rows: int, dim: int,
                     eps: float) -> None:
     """`qwen35::rms_norm` (src/qwen35.rs:2654-2695): out = x * rsqrt(mean(x^2) + eps) * (1 + w)."""
+    if _native.qwen35_rms_norm(rt, x, w, out, out_as_bf16, rows, dim, eps):
+        return
     capi.call("tessl_qwen35_rms_norm", rt.handle, x.c(), w.c(), out.c(), int(out_as_bf16), rows, dim, eps)
 
 
 def qwen35_residual_add(rt: Runtime, y: GpuBuffer, resid: GpuBuffer, rows: int, width: int) -> None:
     """`qwen35::residual_add` for dense operands (src/qwen35.rs:2586-2623): resid += y."""
+    if _native.qwen35_residual_add(rt, y, resid, rows, width):
+        return
     capi.call("tessl_qwen35_residual_add", rt.handle, y.c(), resid.c(), rows, width)
 
 
 def qwen35_add_rms_norm(rt: Runtime, y: GpuBuffer, resid: GpuBuffer, w: GpuBuffer, out: GpuBuffer, out_as_bf16: bool,
                         rows: int, dim: int, eps: float) -> None:
     """`qwen35::add_rms_norm` (src/qwen35.rs:2697-2747): the add and the norm in one launch."""
+    if _native.qwen35_add_rms_norm(rt, y, resid, w, out, out_as_bf16, rows, dim, eps):
+        return
     capi.call("tessl_qwen35_add_rms_norm", rt.handle, y.c(), resid.c(), w.c(), out.c(), int(out_as_bf16), rows, dim, eps)
 
 
