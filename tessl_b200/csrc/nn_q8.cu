@@ -10,7 +10,10 @@
 // 512-column chunks, a lane reads 16 codes per row and chunk with one 128-bit
 // load and all R loads are issued before any is used. Codes become floats by a
 // byte permute into the mantissa of 2^23 and one subtraction (exact).
+#include <algorithm>
+
 #include "q4_common.cuh"
+#include "q4_gemv_tma.cuh"
 #include "runtime.h"
 
 namespace tessl {
@@ -204,6 +207,210 @@ __global__ void __launch_bounds__(128) q8_i8_kernel(const Q8Params p)
     }
 }
 
+// ------------------------------------------------ reference convention, streamed ---
+
+constexpr uint32_t kI8Rows = 4;                  // rows of a stage per team
+constexpr uint32_t kI8Consumers = 16, kI8Threads = (1 + kI8Consumers) * 32;
+constexpr uint32_t kI8MaxStages = 32, kI8Ring = 200 * 1024, kI8StageCodes = 24 * 1024;
+constexpr uint32_t kI8MaxCols = 8192;
+
+struct I8Plan {
+    uint32_t per_row;     // warps that share a row, 512 columns each (or several times 512)
+    uint32_t share;       // groups of such warps (teams) that share a stage, kI8Rows rows for each
+    uint32_t sets;        // sets of `share` teams, which take turns at the stages
+    uint32_t stages;      // a multiple of sets
+    uint32_t stage_bytes;
+    uint32_t row_step;    // rows per block, a multiple of kI8Rows
+    uint32_t *status;
+};
+
+/// Reference-convention Q8 (int8, f32 scale/zero, f32 x): groups and rows of a multiple of 16 columns, tables at 16-byte
+/// boundaries, at most 8192 columns.
+///
+/// HBM-bound in intent (18.9 MB at 4096 x 4096): one block per SM owns a run of rows and a producer warp streams them, ~16 KB at a
+/// time, with three bulk copies (codes, scales, zeros: each contiguous) into a ring of up to 200 KB; 44 KB in flight would cover
+/// bandwidth times latency. Smaller stages pay the copy unit per copy (4 KB at 1024 columns: 14336 rows 11.2 us against 7.3), larger
+/// ones start late (32 KB at 4096 x 4096: 7.9 us against 7.0). Consumer warps keep x in
+/// registers, each lane the 16 columns it has of every row (rows of up to 4096 columns). q8_i8_kernel issues its loads per two or eight rows and waits for them (long-scoreboard stalls, 27 % of the DRAM
+/// rate), and reads x from L1 again for each.
+/// Before (q8_i8_kernel) -> here, back to back: 4096 x 4096 9.6 -> 7.0 us, 14336 x 4096 24.8 -> 17.0 (3.9 TB/s), 14336 x 1024 9.4 -> 6.7, 2048 x
+/// 2560 4.5 -> 3.9, 4096 x 512 5.4 -> 2.6; relative error against 64 bits 1.9e-7 -> 1.1e-7 (signed codes are summed, not codes + 128).
+/// What bounds it now: the FMA and ALU pipes (a byte permute, a subtraction and an FMA per code) and ~2 us of start.
+/// A ring slot belongs to one set of teams, so a parity that a team waits for is never a round behind.
+/// A row's sums are reduced over the lanes, then over the warps in order: its order of summation depends on cols alone.
+__global__ void __launch_bounds__(kI8Threads, 1) q8_i8_stream_kernel(const Q8Params p, const I8Plan plan)
+{
+    extern __shared__ __align__(128) uint8_t ring[];
+    __shared__ __align__(8) uint64_t bars[2 * kI8MaxStages];
+    __shared__ float red[2][kI8Consumers][kI8Rows];
+    __shared__ int abort_flag;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t cols = p.cols, gpr = cols / p.group_size;
+    const uint32_t first = blockIdx.x * plan.row_step, last = min(first + plan.row_step, p.rows);
+    const uint32_t stage_rows = plan.share * kI8Rows, nst = (last - first + stage_rows - 1) / stage_rows;
+    const uint32_t bar0 = q4k::smem_u32(bars), ring0 = q4k::smem_u32(ring);
+    auto full = [&](uint32_t s) { return bar0 + 8 * s; };
+    auto empty = [&](uint32_t s) { return bar0 + 8 * (kI8MaxStages + s); };
+    if (threadIdx.x < plan.stages) {
+        q4k::mbar_init(full(threadIdx.x), 1), q4k::mbar_init(empty(threadIdx.x), plan.share * plan.per_row);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (threadIdx.x == 0) abort_flag = 0;
+    __syncthreads();
+    volatile int *abortp = &abort_flag;
+    auto fail = [&](uint32_t role, uint32_t where) {
+        *abortp = 1;
+        *(volatile uint32_t *)plan.status = (role << 24) | (where & 0xffffffu);
+    };
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const uint32_t off_sc = stage_rows * cols, off_zp = off_sc + stage_rows * gpr * 4;
+
+    if (warp == 0) {
+        uint32_t slot = 0, phase = 0, issued = 0;
+        for (uint32_t st = 0; st < nst; ++st) {
+            if (!q4k::mbar_wait(empty(slot), phase ^ 1u, abortp, 20)) {
+                if (lane == 0) fail(1, st);
+                break;
+            }
+            __syncwarp();
+            const uint32_t row = first + st * stage_rows, rows = min(stage_rows, last - row);
+            const uint32_t dst = ring0 + slot * plan.stage_bytes, code_bytes = rows * cols, tab_bytes = rows * gpr * 4;
+            const size_t g0 = (size_t)row * gpr;
+            const bool whole = tab_bytes % 16 == 0;  // the last rows' tables may not be a whole number of 16 bytes
+            if (!whole) {
+                for (uint32_t i = lane; i < rows * gpr; i += 32) {
+                    asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + off_sc + i * 4), "f"(p.scales[g0 + i]) : "memory");
+                    asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + off_zp + i * 4), "f"(p.zeros[g0 + i]) : "memory");
+                }
+                __syncwarp();
+            }
+            if (lane == 0) {
+                q4k::mbar_expect_tx(full(slot), code_bytes + (whole ? 2 * tab_bytes : 0));
+                q4k::bulk_g2s(dst, p.codes + (size_t)row * cols, code_bytes, full(slot));
+                if (whole) {
+                    q4k::bulk_g2s(dst + off_sc, p.scales + g0, tab_bytes, full(slot));
+                    q4k::bulk_g2s(dst + off_zp, p.zeros + g0, tab_bytes, full(slot));
+                }
+            }
+            ++issued;
+            if (++slot == plan.stages) slot = 0, phase ^= 1u;
+        }
+        if (lane == 0 && *abortp) {  // let what is in flight land before the block may exit
+            const long long t0 = clock64();
+            for (uint32_t i = issued > plan.stages ? issued - plan.stages : 0; i < issued; ++i)
+                while (!q4k::mbar_try(full(i % plan.stages), (i / plan.stages) & 1u))
+                    if (clock64() - t0 > 20000000ll) break;
+        }
+        return;
+    }
+    const uint32_t w = warp - 1, team = w / plan.per_row, part = w - team * plan.per_row;
+    if (team >= plan.share * plan.sets) return;
+    const uint32_t set = team / plan.share, seat = team - set * plan.share;
+    const uint32_t k_first = part * kChunk8 + lane * 16, k_step = plan.per_row * kChunk8, nch = (cols + k_step - 1) / k_step;
+    const float *x = static_cast<const float *>(p.x);
+    float xs[16], xsum = 0.0f;
+    auto load_x = [&](uint32_t k) {
+        xsum = 0.0f;
+#pragma unroll
+        for (uint32_t v = 0; v < 4; ++v) {
+            const uint4 u = k < cols ? dev::ld_after_wait16(x + k + 4 * v) : make_uint4(0, 0, 0, 0);
+            xs[4 * v] = __uint_as_float(u.x), xs[4 * v + 1] = __uint_as_float(u.y);
+            xs[4 * v + 2] = __uint_as_float(u.z), xs[4 * v + 3] = __uint_as_float(u.w);
+            xsum += (xs[4 * v] + xs[4 * v + 1]) + (xs[4 * v + 2] + xs[4 * v + 3]);
+        }
+    };
+    load_x(k_first);
+    uint32_t g = min(k_first, cols - 1) / p.group_size;
+    uint32_t slot = set, phase = 0, parity = 0;
+    bool dead = false;
+    for (uint32_t st = set; st < nst; st += plan.sets, parity ^= 1u) {
+        // After a wait that ran out the team goes on to its barriers, without waiting for copies: no warp is left behind at one.
+        if (!dead && !__all_sync(0xffffffffu, q4k::mbar_wait(full(slot), phase, abortp, 0))) {
+            if (lane == 0) fail(2, st);
+            dead = true;
+        }
+        const uint32_t row0 = first + st * stage_rows + seat * kI8Rows;
+        if (row0 >= last) break;  // the last stage has no rows for this team
+        const uint32_t src = ring0 + slot * plan.stage_bytes, rt0 = seat * kI8Rows;
+        float acc[kI8Rows] = {0.0f, 0.0f, 0.0f, 0.0f};
+        for (uint32_t c = 0; c < nch; ++c) {
+            const uint32_t k = k_first + c * k_step;
+            if (k >= cols) break;  // the bytes there are another row's
+            if (nch > 1) load_x(k), g = k / p.group_size;
+#pragma unroll
+            for (uint32_t r = 0; r < kI8Rows; ++r) {
+                const uint4 q = q4k::lds128(src + (rt0 + r) * cols + k);
+                float sc, zp;
+                asm volatile("ld.shared.f32 %0, [%1];" : "=f"(sc) : "r"(src + off_sc + ((rt0 + r) * gpr + g) * 4) : "memory");
+                asm volatile("ld.shared.f32 %0, [%1];" : "=f"(zp) : "r"(src + off_zp + ((rt0 + r) * gpr + g) * 4) : "memory");
+                // flipping the top bit of each byte gives code + 128 unsigned; it goes again with the 2^23 of the conversion
+                const uint32_t u[4] = {q.x ^ 0x80808080u, q.y ^ 0x80808080u, q.z ^ 0x80808080u, q.w ^ 0x80808080u};
+                float d0 = 0.0f, d1 = 0.0f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    d0 = fmaf(xs[4 * j], byte_to_f2p23<0>(u[j]) - 8388736.0f, d0);
+                    d1 = fmaf(xs[4 * j + 1], byte_to_f2p23<1>(u[j]) - 8388736.0f, d1);
+                    d0 = fmaf(xs[4 * j + 2], byte_to_f2p23<2>(u[j]) - 8388736.0f, d0);
+                    d1 = fmaf(xs[4 * j + 3], byte_to_f2p23<3>(u[j]) - 8388736.0f, d1);
+                }
+                acc[r] = fmaf(sc, fmaf(-zp, xsum, d0 + d1), acc[r]);  // sum x * (q - zero)
+            }
+        }
+        __syncwarp();
+        if (lane == 0) q4k::mbar_arrive(empty(slot));
+        // Lanes: four rows halve to one per lane (lane bits 4 and 3 pick the row), then the other bits.
+#pragma unroll
+        for (int h = kI8Rows / 2; h > 0; h >>= 1) {
+            const bool up = (lane & (8 * h)) != 0;
+#pragma unroll
+            for (int r = 0; r < h; ++r) {
+                const float send = up ? acc[r] : acc[r + h], keep = up ? acc[r + h] : acc[r];
+                acc[r] = keep + __shfl_xor_sync(0xffffffffu, send, 8 * h);
+            }
+        }
+        float v = acc[0];
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (plan.per_row > 1) {
+            if ((lane & 7) == 0) red[parity][w][lane >> 3] = v;
+            // the team's warps; this buffer is written again after the next of these barriers only
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(plan.per_row * 32) : "memory");
+            if (part == 0 && lane < kI8Rows) {
+                v = red[parity][w][lane];
+                for (uint32_t i = 1; i < plan.per_row; ++i) v += red[parity][w + i][lane];
+            }
+        } else {
+            v = __shfl_sync(0xffffffffu, v, (lane & 3) * 8);
+        }
+        const uint32_t row = row0 + lane;
+        if (part == 0 && lane < kI8Rows && row < last) static_cast<float *>(p.y)[row] = v;
+        slot += plan.sets;
+        if (slot >= plan.stages) slot -= plan.stages, phase ^= 1u;
+    }
+}
+
+Result launch_i8_stream(TesslRuntime *rt, const Q8Params &p)
+{
+    I8Plan plan{};
+    const uint32_t chunks = (p.cols + kChunk8 - 1) / kChunk8, gpr = p.cols / p.group_size;
+    plan.per_row = std::min<uint32_t>(chunks, 8u);
+    const uint32_t teams = kI8Consumers / plan.per_row;
+    plan.share = 1;
+    for (uint32_t d = 2; d <= teams; ++d)
+        if (teams % d == 0 && d * kI8Rows * p.cols <= kI8StageCodes) plan.share = d;
+    plan.sets = teams / plan.share;
+    plan.stage_bytes = plan.share * kI8Rows * (p.cols + 8 * gpr);  // a multiple of 16; at most 48 KB
+    plan.stages = std::min<uint32_t>(kI8MaxStages, kI8Ring / plan.stage_bytes) / plan.sets * plan.sets;
+    const uint32_t batches = (p.rows + kI8Rows - 1) / kI8Rows, blocks = std::min<uint32_t>(batches, (uint32_t)rt->sm_count);
+    plan.row_step = (batches + blocks - 1) / blocks * kI8Rows;
+    plan.status = rt->status_dev;
+    const size_t smem = (size_t)plan.stages * plan.stage_bytes;
+    TESSL_TRY(smem_opt_in(rt, reinterpret_cast<const void *>(q8_i8_stream_kernel), smem, "gemv_q8: shared memory opt-in", true));
+    return launch_pdl(rt, "gemv_q8 launch", q8_i8_stream_kernel, dim3((p.rows + plan.row_step - 1) / plan.row_step), dim3(kI8Threads), smem,
+                      p, plan);
+}
+
 /// Any group size and alignment: one warp per row, lanes stride the columns,
 /// w = scale * (q - zero) per element as the reference's scalar path does
 /// (kernels/gemv_q8.metal:101-113).
@@ -267,6 +474,10 @@ Result gemv_q8(TesslRuntime *rt, const TesslBuf &packed, const TesslBuf &scales,
     const bool vec = group_size % 16 == 0 && cols % 16 == 0 && ((uintptr_t)packed.ptr & 15u) == 0 &&
                      ((uintptr_t)x.ptr & 15u) == 0 && cols > 0;
     if (vec) {
+        // The tables of every fourth row start at 16-byte boundaries if the buffers do. Below a megabyte of codes the start of the
+        // ring costs more than it gives: 512 x 1024 2.35 us without it, 2.55 with it; 513 x 4096 3.5 / 2.7.
+        if (cols <= kI8MaxCols && weights >= (1u << 20) && (((uintptr_t)scales.ptr | (uintptr_t)zeros.ptr) & 15u) == 0)
+            return launch_i8_stream(rt, p);
         const int warps = (int)std::max<uint32_t>(1u, std::min<uint32_t>(4u, (cols + kChunk8 - 1) / kChunk8));
         if ((uint64_t)rows >= (uint64_t)(8 * 3 * rt->sm_count)) {
             q8_i8_kernel<8><<<(rows + 7) / 8, warps * 32, 0, rt->stream>>>(p);
