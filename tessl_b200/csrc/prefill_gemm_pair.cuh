@@ -31,6 +31,32 @@
 namespace tessl {
 namespace pf {
 
+/// First K block of a cluster's tile `it` that dequant group `grp` expands; it goes on in steps of NG. Main K blocks are dealt out by
+/// their running index over the cluster's tiles, so a stage of the packed ring (NG divides its depth) belongs to one group: copies may
+/// land out of order, and a group that comes to a stage whose last copy another group still waits for cannot tell that copy's round from
+/// its own. (With a restart at block `grp` in every tile an odd number of main blocks changed the owner, and with one extra block,
+/// SQ + 1 < SA, nothing else promised that the earlier copy had landed: K = 960 in groups of 64 over several 256- or 64-wide tiles.)
+template <int NG>
+__host__ __device__ constexpr uint32_t first_block(uint32_t it, uint32_t nkb_main, uint32_t grp)
+{
+    return (grp + NG - it * nkb_main % NG) % NG;
+}
+template <int NG>
+constexpr bool groups_take_running_indices()
+{
+    for (uint32_t nkb_main = 1; nkb_main <= 2 * NG; ++nkb_main)
+        for (uint32_t it = 0; it <= 2 * NG; ++it) {
+            uint32_t firsts = 0;
+            for (uint32_t grp = 0; grp < NG; ++grp) {
+                const uint32_t kb = first_block<NG>(it, nkb_main, grp);
+                if ((it * nkb_main + kb) % NG != grp) return false;
+                firsts |= 1u << kb;
+            }
+            if (firsts != (1u << NG) - 1) return false;  // every block is somebody's
+        }
+    return true;
+}
+
 template <int BN>
 struct PairCfg {
     static constexpr int HB = BN / 2;                 // weight rows this CTA expands
@@ -38,10 +64,11 @@ struct PairCfg {
     static constexpr int SB = SA;                     // one ring: a K block's two operands are freed together
     static constexpr int SQ = BN == 256 ? 4 : 8;      // packed-W stages
     static constexpr int NDW = HB / 16;               // dequant warps per group (two threads per weight row)
-    static constexpr int NG = 2;                      // dequant groups; group g expands K blocks g, g + 2, ...
-    // A group starts every tile at block g, so its step across the end of a tile is up to 2 NG - 1 blocks; a step longer
-    // than its ring would make the parity that it waits for ambiguous.
-    static_assert(2 * NG - 1 <= SA && 2 * NG - 1 <= SQ, "a dequant group may step past a whole ring");
+    static constexpr int NG = 2;                      // dequant groups, on alternate K blocks
+    static_assert(SQ % NG == 0 && groups_take_running_indices<NG>(), "a packed stage would change hands");
+    // The extra K blocks follow in the same steps, so a group's step across the end of a tile is up to 2 NG - 1 blocks. Stages of the
+    // (X, W) ring are freed in order (one commit each), so there a step of at most the ring keeps the parity unambiguous.
+    static_assert(2 * NG - 1 <= SA, "a dequant group may step past a whole ring");
     static constexpr int FIRST_DW = 8;                // first dequant warp
     static constexpr int THREADS = (FIRST_DW + NG * NDW) * 32;
     // Sleep between mbarrier polls (ns) of the roles that run ahead of the MMA issuer.
@@ -250,7 +277,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<BN>::THREADS
         }
     } else {
         // ------------------------------------------------ dequant warps ---
-        // Group g expands K blocks g, g + 2, ... of this CTA's BN/2 weight rows, two
+        // A group expands every NG-th K block of this CTA's BN/2 weight rows, two
         // threads per row: 16 packed bytes -> 32 f16 values each. The (scale, bias) word
         // of a block is fetched two blocks of this group ahead, right after a block was
         // handed over, so that no global load is still outstanding when the thread
@@ -267,12 +294,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<BN>::THREADS
             const uint32_t n = min((t / p.tiles_m) * BN + rank * C::HB + r, p.N - 1);  // rows past N repeat the last
             const uint32_t *sbrow = p.sb + (size_t)n * p.gpr;
             auto scale_word = [&](uint32_t kb) { return __ldg(sbrow + min((kb * 64 + h * 32) >> p.gshift, p.gpr - 1)); };
-            uint32_t cur = scale_word(grp), nxt = scale_word(grp + C::NG);
+            const uint32_t kb0 = first_block<C::NG>(it, p.nkb_main, grp);
+            uint32_t cur = scale_word(kb0), nxt = scale_word(kb0 + C::NG);
             RingPos<C::SA> ring;   // stage of K block kb of this tile
             RingPos<C::SQ> qring;  // packed stage of that block
-            ring.set(it * nkb + grp);
-            qring.set(it * p.nkb_main + grp);
-            for (uint32_t kb = grp; kb < nkb; kb += C::NG) {
+            ring.set(it * nkb + kb0);
+            qring.set(it * p.nkb_main + kb0);
+            for (uint32_t kb = kb0; kb < nkb; kb += C::NG) {
                 if (!mbar_wait(empty(ring.stage), ring.phase ^ 1u, abortp, C::POLL_DEQUANT)) {
                     if (lane == 0) fail(6, kb);
                     ok_ = false;

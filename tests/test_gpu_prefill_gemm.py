@@ -242,6 +242,34 @@ def test_every_compiled_tile_on_ragged_shapes(rt, tile, pair):
         rt.set_prefill_tile(100, -1)
 
 
+@pytest.mark.parametrize("tile", [64, 128, 192, 256])
+@pytest.mark.parametrize("k,group", [(960, 64), (448, 32), (192, 64), (64, 64)])
+def test_dequant_groups_keep_their_stages_across_tiles(rt, tile, k, group):
+    """An odd number of main K blocks and a single extra one, several tiles per cluster: the dequant groups' order changes from tile to
+    tile, so that every packed stage stays with its group (prefill_gemm_pair.cuh asserts it). Every output through its sums, rows on both
+    sides of the tiles' boundaries against the exact product, the same bits in every pass."""
+    m, n = 700, 10100
+    packed, sb = synth.q4_bank(0x7E553700 + k, n, k, group)
+    packed, sb = packed.view(np.uint8).reshape(-1), sb.reshape(-1)
+    x = synth.normal_bf16(0x7E553707 + k, m * k)
+    bank, xb, y, shape = upload_bank(rt, packed, sb), rt.buffer_from(x), seeded_f32(rt, m * n), nn.QuantShape(n, k, group)
+    rt.set_prefill_tile(tile, 1)
+    try:
+        first = None
+        for _ in range(8):
+            nn.gemm_q4_mlx_tensorops(rt, bank, xb, y, shape, m)
+            got = y.read(np.float32, m * n).reshape(m, n)
+            first = got if first is None else first
+            assert np.array_equal(got.view(np.uint32), first.view(np.uint32))
+    finally:
+        rt.set_prefill_tile(0, -1)
+    assert rt.last_prefill_tile() == (tile, 1)
+    _check_rows_against_the_oracle(got, packed, sb, x, _subset_rows(m), n, k, group, f"tile {tile} K {k}")
+    _check_sums_against_the_oracle(got, packed, sb, x, m, n, k, group, f"tile {tile} K {k}")
+    for b in (bank.packed, bank.scales_biases, xb, y):
+        b.free()
+
+
 def test_rows_of_any_magnitude_survive_the_f16_operands(rt):
     """The per-row power-of-two rescale: rows scaled by 2^-40 .. 2^+60 give the
     correspondingly scaled outputs, a zero row gives zeros."""
