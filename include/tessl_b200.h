@@ -134,12 +134,22 @@ TESSL_API int32_t tessl_runtime_poison_for_test(TesslRuntime *rt);
  * estimate; 64 with pair = 1 only), pair = 1 / 0 forces the two-CTA or the single-CTA kernel (-1 = the
  * library decides). tessl_runtime_last_prefill_tile reports what the most
  * recent prefill call launched (tile_n = 0 if it ran no tile kernel; 64 with
- * pair = 1 stands for the narrow ones: the 64-wide tile, and the kernel that
- * divides K over a cluster, which the library alone chooses). No
+ * pair = 1 stands for the narrow ones: the 64-wide tile, and the kernel for few
+ * rows of X, which tessl_runtime_last_prefill_split tells apart). No
  * counterpart in the reference, whose kernel has one 32 x 32 tile. */
 TESSL_API int32_t tessl_runtime_set_prefill_tile(TesslRuntime *rt, uint32_t tile_n, int32_t pair, char *err, size_t err_len);
 TESSL_API int32_t tessl_runtime_last_prefill_tile(TesslRuntime *rt, uint32_t *tile_n, uint32_t *pair, char *err,
                                         size_t err_len);
+
+/* The prefill kernel for few rows of X, which divides K over the CTAs of a
+ * cluster: split = 1 .. 6 makes later tessl_gemm_q4_mlx_tensorops* calls run it
+ * with that many CTAs per tile (before any choice of tessl_runtime_set_prefill_tile;
+ * a call whose K has fewer than four blocks of 64 columns for each is refused),
+ * 0 keeps them from it, -1 lets the library decide.
+ * tessl_runtime_last_prefill_split reports the CTAs per tile of the most recent
+ * prefill call, 0 if it ran another kernel. */
+TESSL_API int32_t tessl_runtime_set_prefill_split(TesslRuntime *rt, int32_t split, char *err, size_t err_len);
+TESSL_API int32_t tessl_runtime_last_prefill_split(TesslRuntime *rt, uint32_t *split, char *err, size_t err_len);
 
 /* Clock budget (SM clocks) of the bounded waits a kernel of this runtime makes
  * on another GPU's flags (tessl_peer_gather and the sharded GEMV's exchange);

@@ -274,6 +274,28 @@ int32_t tessl_runtime_last_prefill_tile(TesslRuntime *rt, uint32_t *tile_n, uint
     return TESSL_OK;
 }
 
+int32_t tessl_runtime_set_prefill_split(TesslRuntime *rt, int32_t split, char *err, size_t err_len)
+{
+    if (refuse_unowned(rt, err, err_len)) return TESSL_ERR;
+    if (split < -1 || split > 6) {
+        write_err(err, err_len, tessl::fmt("tessl_runtime_set_prefill_split: split %d is outside -1 .. 6", split));
+        return TESSL_ERR;
+    }
+    rt->prefill_force_split = split;
+    return TESSL_OK;
+}
+
+int32_t tessl_runtime_last_prefill_split(TesslRuntime *rt, uint32_t *split, char *err, size_t err_len)
+{
+    if (refuse_unowned(rt, err, err_len)) return TESSL_ERR;
+    if (!split) {
+        write_err(err, err_len, "tessl_runtime_last_prefill_split: null out");
+        return TESSL_ERR;
+    }
+    *split = (uint32_t)rt->prefill_last_split;
+    return TESSL_OK;
+}
+
 int32_t tessl_runtime_set_peer_wait_limit(TesslRuntime *rt, uint64_t clocks, char *err, size_t err_len)
 {
     if (refuse_unowned(rt, err, err_len)) return TESSL_ERR;

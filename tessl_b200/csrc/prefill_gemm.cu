@@ -552,6 +552,12 @@ Result split_plan(TesslRuntime *rt, uint32_t m, const PrefillPlan &pl, SplitPlan
     const uint32_t x_rows = ((m + tiles_m - 1) / tiles_m + 15) & ~15u;
     const uint64_t tiles = (uint64_t)tiles_m * ((pl.n + SplitCfg::ROWS - 1) / SplitCfg::ROWS);
     const uint32_t blocks = pl.nkb_main + pl.nkb_extra;
+    if (rt->prefill_force_split > 0) {
+        const uint32_t s = (uint32_t)rt->prefill_force_split;
+        if (blocks < 4 * s) return fmt("%s: K = %u has %u blocks, a split over %u CTAs takes %u", kWhat, pl.k, blocks, s, 4 * s);
+        best = SplitPlan{tiles_m, x_rows, s, 0};
+        return ok();
+    }
     for (uint32_t s = 1; s <= kSplitMaxUsed && blocks >= 4 * s; ++s) {
         const uint64_t room = (uint64_t)split_clusters(rt, s), waves = (tiles + room - 1) / room;
         const uint64_t part = (blocks + s - 1) / s;
@@ -625,6 +631,8 @@ Result prefill_launch(TesslRuntime *rt, const TesslQ4MlxBank &bank, const TesslB
 {
     __half *a_aug = static_cast<__half *>(scratch);
     float *row_scale = reinterpret_cast<float *>(static_cast<char *>(scratch) + pl.a_bytes);
+    SplitPlan sp;
+    if (rt->prefill_force_split > 0) TESSL_TRY(split_plan(rt, m, pl, &sp));  // may refuse: before any launch
     const uint32_t chunks = pl.k64 / 8, per = (chunks + kPrepMaxThreads - 1) / kPrepMaxThreads;  // chunks per thread
     const auto prep = per == 1 ? x_prepare_kernel<1> : per == 2 ? x_prepare_kernel<2> : x_prepare_kernel<0>;
     const uint32_t threads = per > 2 ? kPrepMaxThreads : ((chunks + per - 1) / per + 31) & ~31u;
@@ -634,21 +642,22 @@ Result prefill_launch(TesslRuntime *rt, const TesslQ4MlxBank &bank, const TesslB
     TESSL_TRY(launch_pdl(rt, "gemm_q4_mlx_tensorops pre-pass launch", prep, dim3(m), dim3(threads), 0,
                          static_cast<const uint16_t *>(x_bf16.ptr), a_aug, row_scale, pl.k, pl.k64, pl.k_aug, pl.gshift));
 
+    auto run_split = [&] {
+        rt->prefill_last_bn = 64, rt->prefill_last_pair = 1, rt->prefill_last_split = (int)sp.split;
+        return launch_gemm_split(rt, bank, y, m, out, pl, sp, a_aug, row_scale);
+    };
+    if (sp.split) return run_split();
     const bool pair = rt->sm_count >= 2 && rt->prefill_force_pair != 0;
     const uint32_t tiles_m = pair ? (m + 2 * BM - 1) / (2 * BM) : (m + BM - 1) / BM;
     const int bn = rt->prefill_force_bn
                        ? rt->prefill_force_bn
                        : pick_tile_width(tiles_m, pl.n, pair ? (uint32_t)rt->sm_count / 2 : (uint32_t)rt->sm_count, pair);
-    if (rt->prefill_force_bn == 0 && rt->prefill_force_pair < 0 && pair) {
-        SplitPlan sp;
+    if (rt->prefill_force_split < 0 && rt->prefill_force_bn == 0 && rt->prefill_force_pair < 0 && pair) {
         TESSL_TRY(split_plan(rt, m, pl, &sp));
         // Split kernel / pair kernel, us: 25 x 4096 x 4096 11.2 / 19.1, 509 x 2048 x 6144 23.4 / 30.4, 320 x 9216 x 2048 16.5 / 22.3,
         // 509 x 3072 x 2048 14.4 / 15.4; and the other way: 200 x 12288 x 4096 41.2 / 29.4, 509 x 4096 x 1024 10.8 / 10.5, 420 x 3072 x
         // 1024 10.8 / 10.2. The 3 % are for shapes where the estimates meet.
-        if (sp.cost * 100 < pair_cost(m, pl, bn, (uint32_t)rt->sm_count / 2) * 97) {
-            rt->prefill_last_bn = 64, rt->prefill_last_pair = 1;
-            return launch_gemm_split(rt, bank, y, m, out, pl, sp, a_aug, row_scale);
-        }
+        if (sp.cost * 100 < pair_cost(m, pl, bn, (uint32_t)rt->sm_count / 2) * 97) return run_split();
     }
     rt->prefill_last_bn = bn, rt->prefill_last_pair = pair ? 1 : 0;
 
@@ -735,8 +744,8 @@ Result gemm_q4_mlx_tensorops(TesslRuntime *rt, const TesslQ4MlxBank &bank, const
     bool empty = false;
     TESSL_TRY(prefill_validate(bank, x_bf16, y, shape, m, out, &pl, &empty));
     if (empty) return ok();
-    rt->prefill_last_bn = 0, rt->prefill_last_pair = 0;
-    if (rt->prefill_force_bn == 0 && rt->prefill_force_pair < 0) {
+    rt->prefill_last_bn = 0, rt->prefill_last_pair = 0, rt->prefill_last_split = 0;
+    if (rt->prefill_force_bn == 0 && rt->prefill_force_pair < 0 && rt->prefill_force_split < 1) {
         bool handled = false;  // a few rows: batches of 8 on the tensor-core GEMV kernel
         TESSL_TRY(prefill_as_small_batches(rt, bank, x_bf16, y, shape, m, out, &handled));
         if (handled) return ok();
@@ -769,8 +778,8 @@ Result gemm_q4_mlx_tensorops_noalloc(TesslRuntime *rt, const TesslQ4MlxBank &ban
     bool empty = false;
     TESSL_TRY(prefill_validate(bank, x_bf16, y, shape, m, out, &pl, &empty));
     if (empty) return ok();
-    rt->prefill_last_bn = 0, rt->prefill_last_pair = 0;
-    if (rt->prefill_force_bn == 0 && rt->prefill_force_pair < 0) {
+    rt->prefill_last_bn = 0, rt->prefill_last_pair = 0, rt->prefill_last_split = 0;
+    if (rt->prefill_force_bn == 0 && rt->prefill_force_pair < 0 && rt->prefill_force_split < 1) {
         bool handled = false;  // needs no scratch at all
         TESSL_TRY(prefill_as_small_batches(rt, bank, x_bf16, y, shape, m, out, &handled));
         if (handled) return ok();

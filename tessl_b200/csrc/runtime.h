@@ -65,6 +65,9 @@ struct TesslRuntime {
     int prefill_force_pair = -1;
     int prefill_last_bn = 0;
     int prefill_last_pair = 0;
+    // The same for the split kernel: CTAs per tile (0 = not that kernel, -1 = the library decides).
+    int prefill_force_split = -1;
+    int prefill_last_split = 0;
     // Clock budget of a bounded device-side wait on another rank (0 = the default).
     uint64_t peer_wait_clocks = 0;
 };

@@ -185,6 +185,17 @@ class Runtime:
         capi.call("tessl_runtime_last_prefill_tile", self.handle, C.byref(bn), C.byref(pair))
         return bn.value, pair.value
 
+    def set_prefill_split(self, split: int = -1) -> None:
+        """Make later prefill GEMM calls run the kernel that divides K over a cluster, with `split` CTAs per tile (1 .. 6), keep them
+        from it (0), or let the library decide (-1)."""
+        capi.call("tessl_runtime_set_prefill_split", self.handle, split)
+
+    def last_prefill_split(self) -> int:
+        """CTAs per tile of that kernel in the most recent prefill GEMM call; 0 if another one ran."""
+        split = C.c_uint32(0)
+        capi.call("tessl_runtime_last_prefill_split", self.handle, C.byref(split))
+        return split.value
+
     def set_peer_wait_limit(self, clocks: int) -> None:
         """Clock budget of bounded waits on another GPU's flags (0 = the default, about 0.5 s)."""
         capi.call("tessl_runtime_set_peer_wait_limit", self.handle, clocks)

@@ -1,5 +1,6 @@
 """The 64-wide tile of the CTA-pair prefill GEMM, which the library picks when wider tiles would leave clusters idle: ragged
-edges in both directions, every group size, f32 and bf16, against the exact product."""
+edges in both directions, every group size, f32 and bf16, against the exact product. Some of these shapes are the split
+kernel's by choice; they are kept from it here."""
 import numpy as np
 import pytest
 
@@ -8,6 +9,13 @@ from oracle import api
 from tessl_b200 import nn, synth
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def _pair_kernel(rt):
+    rt.set_prefill_split(0)
+    yield
+    rt.set_prefill_split(-1)
 
 
 @pytest.mark.parametrize("m,n,k,group", [(77, 4096, 1536, 64), (33, 65, 2080, 32), (25, 300, 4224, 128), (257, 1999, 1088, 64),
@@ -19,7 +27,7 @@ def test_narrow_tiles_match_the_exact_product(rt, m, n, k, group):
     bank, xb, shape = upload_bank(rt, packed, sb), rt.buffer_from(x), nn.QuantShape(n, k, group)
     y = seeded_f32(rt, m * n, 256)
     nn.gemm_q4_mlx_tensorops(rt, bank, xb, y, shape, m)
-    assert rt.last_prefill_tile() == (64, 1)
+    assert rt.last_prefill_tile() == (64, 1) and rt.last_prefill_split() == 0
     out = y.read(np.float32, m * n + 256)
     assert np.all(out[m * n:] == SENTINEL_F32), "wrote past y"
     got = out[: m * n].reshape(m, n)
@@ -53,7 +61,7 @@ def test_several_narrow_tiles_per_cluster(rt, m, n, k, group, forced):
         nn.gemm_q4_mlx_tensorops(rt, bank, xb, y, shape, m)
     finally:
         rt.set_prefill_tile(0, -1)
-    assert rt.last_prefill_tile() == (64, 1)
+    assert rt.last_prefill_tile() == (64, 1) and rt.last_prefill_split() == 0
     out = y.read(np.float32, m * n + 1024)
     assert np.all(out[m * n:] == SENTINEL_F32), "wrote past y"
     got = out[: m * n].reshape(m, n)
