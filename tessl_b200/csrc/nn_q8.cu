@@ -140,10 +140,37 @@ __global__ void __launch_bounds__(128) q8_mlx_kernel(const Q8Params p)
     }
 }
 
+// ------------------------------------------------------- reference convention ---
+
+constexpr uint32_t kI8MaxCols = 8192;  // of the streamed kernel
+
+/// Warps that share a row, 512 columns each or several times 512. The order of a row's sums is a function of cols alone, in both
+/// kernels, so a slice of a bank has the bits of the whole, wherever its tables lie.
+uint32_t i8_warps_per_row(uint32_t cols)
+{
+    return std::min((cols + kChunk8 - 1) / kChunk8, cols > kI8MaxCols ? 4u : 8u);  // beyond the streamed kernel's rows, four
+}
+
+/// A lane's 16 signed codes of a row against its columns of x, added to `acc` with the group's scale and zero.
+__device__ __forceinline__ void i8_dot16(const uint4 &q, const float (&xs)[16], float xsum, float scale, float zero, float &acc)
+{
+    // flipping the top bit of each byte gives code + 128 unsigned; it goes again with the 2^23 of the conversion
+    const uint32_t u[4] = {q.x ^ 0x80808080u, q.y ^ 0x80808080u, q.z ^ 0x80808080u, q.w ^ 0x80808080u};
+    float d0 = 0.0f, d1 = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        d0 = fmaf(xs[4 * j], byte_to_f2p23<0>(u[j]) - 8388736.0f, d0);
+        d1 = fmaf(xs[4 * j + 1], byte_to_f2p23<1>(u[j]) - 8388736.0f, d1);
+        d0 = fmaf(xs[4 * j + 2], byte_to_f2p23<2>(u[j]) - 8388736.0f, d0);
+        d1 = fmaf(xs[4 * j + 3], byte_to_f2p23<3>(u[j]) - 8388736.0f, d1);
+    }
+    acc = fmaf(scale, fmaf(-zero, xsum, d0 + d1), acc);  // sum x * (q - zero)
+}
+
 /// Reference-convention Q8 (int8, f32 scale/zero, f32 x), vector path: needs
 /// group_size and cols multiples of 16 so a lane's 16 codes share one group.
-template <int R>
-__global__ void __launch_bounds__(128) q8_i8_kernel(const Q8Params p)
+template <int R, int THREADS>
+__global__ void __launch_bounds__(THREADS) q8_i8_kernel(const Q8Params p)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const uint32_t rows = p.rows, cols = p.cols;
@@ -175,24 +202,9 @@ __global__ void __launch_bounds__(128) q8_i8_kernel(const Q8Params p)
             xsum += (xv.x + xv.y) + (xv.z + xv.w);
         }
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            // Signed codes: flipping the top bit of each byte gives code + 128 unsigned.
-            uint4 u = wq[r];
-            u.x ^= 0x80808080u, u.y ^= 0x80808080u, u.z ^= 0x80808080u, u.w ^= 0x80808080u;
-            float q[16];
-            codes16(u, q);
-            float d0 = 0.0f, d1 = 0.0f;
-#pragma unroll
-            for (int i = 0; i < 16; i += 2) {
-                d0 = fmaf(xs[i], q[i], d0);
-                d1 = fmaf(xs[i + 1], q[i + 1], d1);
-            }
-            // sum x * (q + 128 - 128 - zero) = dot - (128 + zero) * xsum
-            const float dot = fmaf(-(128.0f + zp[r]), xsum, d0 + d1);
-            acc[r] = fmaf(sc[r], dot, acc[r]);
-        }
+        for (int r = 0; r < R; ++r) i8_dot16(wq[r], xs, xsum, sc[r], zp[r], acc[r]);
     }
-    __shared__ float red[4][R];
+    __shared__ float red[THREADS / 32][R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const float v = dev::warp_sum(acc[r]);
@@ -212,7 +224,6 @@ __global__ void __launch_bounds__(128) q8_i8_kernel(const Q8Params p)
 constexpr uint32_t kI8Rows = 4;                  // rows of a stage per team
 constexpr uint32_t kI8Consumers = 16, kI8Threads = (1 + kI8Consumers) * 32;
 constexpr uint32_t kI8MaxStages = 32, kI8Ring = 200 * 1024, kI8StageCodes = 24 * 1024;
-constexpr uint32_t kI8MaxCols = 8192;
 
 struct I8Plan {
     uint32_t per_row;     // warps that share a row, 512 columns each (or several times 512)
@@ -227,17 +238,18 @@ struct I8Plan {
 /// Reference-convention Q8 (int8, f32 scale/zero, f32 x): groups and rows of a multiple of 16 columns, tables at 16-byte
 /// boundaries, at most 8192 columns.
 ///
-/// HBM-bound in intent (18.9 MB at 4096 x 4096): one block per SM owns a run of rows and a producer warp streams them, ~16 KB at a
+/// HBM-bound in intent (18.9 MB at 4096 x 4096): one block per SM owns a run of rows and a producer warp streams them, about 16 KB at a
 /// time, with three bulk copies (codes, scales, zeros: each contiguous) into a ring of up to 200 KB; 44 KB in flight would cover
 /// bandwidth times latency. Smaller stages pay the copy unit per copy (4 KB at 1024 columns: 14336 rows 11.2 us against 7.3), larger
-/// ones start late (32 KB at 4096 x 4096: 7.9 us against 7.0). Consumer warps keep x in
-/// registers, each lane the 16 columns it has of every row (rows of up to 4096 columns). q8_i8_kernel issues its loads per two or eight rows and waits for them (long-scoreboard stalls, 27 % of the DRAM
-/// rate), and reads x from L1 again for each.
-/// Before (q8_i8_kernel) -> here, back to back: 4096 x 4096 9.6 -> 7.0 us, 14336 x 4096 24.8 -> 17.0 (3.9 TB/s), 14336 x 1024 9.4 -> 6.7, 2048 x
-/// 2560 4.5 -> 3.9, 4096 x 512 5.4 -> 2.6; relative error against 64 bits 1.9e-7 -> 1.1e-7 (signed codes are summed, not codes + 128).
+/// ones start late (32 KB at 4096 x 4096: 7.9 us against 7.0). Consumer warps keep x in registers, each lane the 16 columns it has of
+/// every row (rows of up to 4096 columns). q8_i8_kernel issues its loads per two or eight rows and waits for them, and reads x from
+/// L1 again for each.
+/// Before (q8_i8_kernel) -> here, back to back: 4096 x 4096 9.6 -> 7.0 us, 14336 x 4096 24.8 -> 17.0 (3.9 TB/s), 14336 x 1024 9.4 -> 6.7,
+/// 2048 x 2560 4.5 -> 3.9, 4096 x 512 5.4 -> 2.6; relative error against 64 bits 1.9e-7 -> 1.1e-7 (signed codes
+/// are summed, not codes + 128).
 /// What bounds it now: the FMA and ALU pipes (a byte permute, a subtraction and an FMA per code) and ~2 us of start.
 /// A ring slot belongs to one set of teams, so a parity that a team waits for is never a round behind.
-/// A row's sums are reduced over the lanes, then over the warps in order: its order of summation depends on cols alone.
+/// A row's sums are reduced over the lanes, then over the warps in order.
 __global__ void __launch_bounds__(kI8Threads, 1) q8_i8_stream_kernel(const Q8Params p, const I8Plan plan)
 {
     extern __shared__ __align__(128) uint8_t ring[];
@@ -344,17 +356,7 @@ __global__ void __launch_bounds__(kI8Threads, 1) q8_i8_stream_kernel(const Q8Par
                 float sc, zp;
                 asm volatile("ld.shared.f32 %0, [%1];" : "=f"(sc) : "r"(src + off_sc + ((rt0 + r) * gpr + g) * 4) : "memory");
                 asm volatile("ld.shared.f32 %0, [%1];" : "=f"(zp) : "r"(src + off_zp + ((rt0 + r) * gpr + g) * 4) : "memory");
-                // flipping the top bit of each byte gives code + 128 unsigned; it goes again with the 2^23 of the conversion
-                const uint32_t u[4] = {q.x ^ 0x80808080u, q.y ^ 0x80808080u, q.z ^ 0x80808080u, q.w ^ 0x80808080u};
-                float d0 = 0.0f, d1 = 0.0f;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    d0 = fmaf(xs[4 * j], byte_to_f2p23<0>(u[j]) - 8388736.0f, d0);
-                    d1 = fmaf(xs[4 * j + 1], byte_to_f2p23<1>(u[j]) - 8388736.0f, d1);
-                    d0 = fmaf(xs[4 * j + 2], byte_to_f2p23<2>(u[j]) - 8388736.0f, d0);
-                    d1 = fmaf(xs[4 * j + 3], byte_to_f2p23<3>(u[j]) - 8388736.0f, d1);
-                }
-                acc[r] = fmaf(sc, fmaf(-zp, xsum, d0 + d1), acc[r]);  // sum x * (q - zero)
+                i8_dot16(q, xs, xsum, sc, zp, acc[r]);
             }
         }
         __syncwarp();
@@ -393,8 +395,8 @@ __global__ void __launch_bounds__(kI8Threads, 1) q8_i8_stream_kernel(const Q8Par
 Result launch_i8_stream(TesslRuntime *rt, const Q8Params &p)
 {
     I8Plan plan{};
-    const uint32_t chunks = (p.cols + kChunk8 - 1) / kChunk8, gpr = p.cols / p.group_size;
-    plan.per_row = std::min<uint32_t>(chunks, 8u);
+    const uint32_t gpr = p.cols / p.group_size;
+    plan.per_row = i8_warps_per_row(p.cols);
     const uint32_t teams = kI8Consumers / plan.per_row;
     plan.share = 1;
     for (uint32_t d = 2; d <= teams; ++d)
@@ -475,14 +477,17 @@ Result gemv_q8(TesslRuntime *rt, const TesslBuf &packed, const TesslBuf &scales,
                      ((uintptr_t)x.ptr & 15u) == 0 && cols > 0;
     if (vec) {
         // The tables of every fourth row start at 16-byte boundaries if the buffers do. Below a megabyte of codes the start of the
-        // ring costs more than it gives: 512 x 1024 2.35 us without it, 2.55 with it; 513 x 4096 3.5 / 2.7.
+        // ring costs more than it gives: 512 x 1024 2.35 us without it, 2.55 with it; 513 x 4096 2.8 / 2.6.
+        const uint32_t warps = i8_warps_per_row(cols);
         if (cols <= kI8MaxCols && weights >= (1u << 20) && (((uintptr_t)scales.ptr | (uintptr_t)zeros.ptr) & 15u) == 0)
             return launch_i8_stream(rt, p);
-        const int warps = (int)std::max<uint32_t>(1u, std::min<uint32_t>(4u, (cols + kChunk8 - 1) / kChunk8));
+        // Blocks of up to four warps have instantiations of their own: with a bound of 256 threads the compiler schedules the loop
+        // differently, and 21 x 12288 took 4.4 us instead of 4.2.
+        auto go = [&](auto kernel, uint32_t r) { kernel<<<(rows + r - 1) / r, warps * 32, 0, rt->stream>>>(p); };
         if ((uint64_t)rows >= (uint64_t)(8 * 3 * rt->sm_count)) {
-            q8_i8_kernel<8><<<(rows + 7) / 8, warps * 32, 0, rt->stream>>>(p);
+            warps <= 4 ? go(q8_i8_kernel<8, 128>, 8) : go(q8_i8_kernel<8, 256>, 8);
         } else {
-            q8_i8_kernel<2><<<(rows + 1) / 2, warps * 32, 0, rt->stream>>>(p);
+            warps <= 4 ? go(q8_i8_kernel<2, 128>, 2) : go(q8_i8_kernel<2, 256>, 2);
         }
     } else {
         q8_i8_scalar_kernel<<<(rows + 3) / 4, 128, 0, rt->stream>>>(p);

@@ -1,5 +1,6 @@
 """`gemv_q8` over the streamed kernel's plans: one to eight warps per row, one set of teams or several, rows of more than 4096 columns, a last
-stage of one to three rows whose tables are no whole number of 16 bytes, and the shapes either side of its domain."""
+stage of one to three rows whose tables are no whole number of 16 bytes, the shapes either side of its domain, and the same bits of a row
+on either side."""
 import numpy as np
 import pytest
 
@@ -42,11 +43,25 @@ def test_streamed_plans(rt, rows, cols, group):
     _check(rt, q, scales, zeros, x, rows, cols, group, rt.buffer_from(scales), rt.buffer_from(zeros))
 
 
-def test_tables_at_a_four_byte_boundary(rt):
-    rows, cols, group = 300, 4096, 64
+def _bits(rt, q, scales, zeros, x, rows, cols, group, offset=0):
+    tables = []
+    for t in (scales, zeros):
+        b = rt.alloc_buffer(t.nbytes + offset)
+        b.write(t, offset)
+        tables.append(b.view(offset, t.nbytes))
+    return _check(rt, q, scales, zeros, x, rows, cols, group, *tables).view(np.uint32)
+
+
+@pytest.mark.parametrize("rows,cols,group", [(66000, 16, 16), (6000, 192, 64), (2731, 384, 128), (1400, 768, 32), (1200, 1280, 64),
+                                             (1000, 1536, 64), (600, 2176, 64), (400, 3072, 64), (300, 4096, 64), (600, 4608, 64),
+                                             (500, 5120, 64), (400, 6144, 64), (400, 6672, 16), (300, 8192, 64), (300, 8208, 16)])
+def test_a_row_has_the_same_bits_in_every_bank(rt, rows, cols, group):
+    """The whole bank through the ring, its tables at an address that is no multiple of 16, and slices below the ring's least size."""
     q, scales, zeros, x = _inputs(rows, cols, group)
-    big = rt.alloc_buffer(scales.nbytes + 4)
-    big.write(scales, 4)
-    a = _check(rt, q, scales, zeros, x, rows, cols, group, rt.buffer_from(scales), rt.buffer_from(zeros))
-    b = _check(rt, q, scales, zeros, x, rows, cols, group, big.view(4, scales.nbytes), rt.buffer_from(zeros))
-    np.testing.assert_allclose(a, b, rtol=1e-4, atol=1e-4)
+    whole = _bits(rt, q, scales, zeros, x, rows, cols, group)
+    assert np.array_equal(whole, _bits(rt, q, scales, zeros, x, rows, cols, group, offset=4))
+    gpr = cols // group
+    for first, n in ((0, 5), (rows - 7, 7), (rows // 2, 64)):
+        part = _bits(rt, q[first * cols:(first + n) * cols], scales[first * gpr:(first + n) * gpr], zeros[first * gpr:(first + n) * gpr], x,
+                     n, cols, group)
+        assert np.array_equal(whole[first:first + n], part)
