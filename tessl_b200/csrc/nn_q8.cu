@@ -145,10 +145,13 @@ __global__ void __launch_bounds__(128) q8_mlx_kernel(const Q8Params p)
 constexpr uint32_t kI8MaxCols = 8192;  // of the streamed kernel
 
 /// Warps that share a row, 512 columns each or several times 512. The order of a row's sums is a function of cols alone, in both
-/// kernels, so a slice of a bank has the bits of the whole, wherever its tables lie.
+/// kernels, so a slice of a bank has the bits of the whole, wherever its tables lie. Above 4096 columns the warps walk the row in even
+/// rounds: with eight at nine chunks the second round would leave seven idle (1820 x 4608 6.3 us with eight, 5.6 with five; 7281 x 4608
+/// 16.0 / 12.8; 1365 x 7168 5.4 with eight, 5.3 with seven).
 uint32_t i8_warps_per_row(uint32_t cols)
 {
-    return std::min((cols + kChunk8 - 1) / kChunk8, cols > kI8MaxCols ? 4u : 8u);  // beyond the streamed kernel's rows, four
+    const uint32_t chunks = (cols + kChunk8 - 1) / kChunk8, rounds = (chunks + 7) / 8;
+    return cols > kI8MaxCols ? 4 : (chunks + rounds - 1) / rounds;  // beyond the streamed kernel's rows
 }
 
 /// A lane's 16 signed codes of a row against its columns of x, added to `acc` with the group's scale and zero.
@@ -223,7 +226,7 @@ __global__ void __launch_bounds__(THREADS) q8_i8_kernel(const Q8Params p)
 
 constexpr uint32_t kI8Rows = 4;                  // rows of a stage per team
 constexpr uint32_t kI8Consumers = 16, kI8Threads = (1 + kI8Consumers) * 32;
-constexpr uint32_t kI8MaxStages = 32, kI8Ring = 200 * 1024, kI8StageCodes = 24 * 1024;
+constexpr uint32_t kI8MaxStages = 32, kI8Ring = 200 * 1024, kI8StageMin = 8 * 1024, kI8StageBest = 16 * 1024, kI8StageMax = 24 * 1024;
 
 struct I8Plan {
     uint32_t per_row;     // warps that share a row, 512 columns each (or several times 512)
@@ -245,9 +248,10 @@ struct I8Plan {
 /// every row (rows of up to 4096 columns). q8_i8_kernel issues its loads per two or eight rows and waits for them, and reads x from
 /// L1 again for each.
 /// Before (q8_i8_kernel) -> here, back to back: 4096 x 4096 9.6 -> 7.0 us, 14336 x 4096 24.8 -> 17.0 (3.9 TB/s), 14336 x 1024 9.4 -> 6.7,
-/// 2048 x 2560 4.5 -> 3.9, 4096 x 512 5.4 -> 2.6; relative error against 64 bits 1.9e-7 -> 1.1e-7 (signed codes
+/// 2048 x 2560 4.5 -> 3.9, 4096 x 512 5.4 -> 2.6, 21845 x 1536 15.0 -> 11.9; relative error against 64 bits 1.9e-7 -> 1.1e-7 (signed codes
 /// are summed, not codes + 128).
-/// What bounds it now: the FMA and ALU pipes (a byte permute, a subtraction and an FMA per code) and ~2 us of start.
+/// What bounds it now: the FMA and ALU pipes (a byte permute, a subtraction and an FMA per code) and ~2 us of start. Rows dealt out
+/// one by one instead of four by four change nothing or lose (2048 x 4096 4.65 -> 4.9): a block's time goes by its stages.
 /// A ring slot belongs to one set of teams, so a parity that a team waits for is never a round behind.
 /// A row's sums are reduced over the lanes, then over the warps in order.
 __global__ void __launch_bounds__(kI8Threads, 1) q8_i8_stream_kernel(const Q8Params p, const I8Plan plan)
@@ -398,10 +402,16 @@ Result launch_i8_stream(TesslRuntime *rt, const Q8Params &p)
     const uint32_t gpr = p.cols / p.group_size;
     plan.per_row = i8_warps_per_row(p.cols);
     const uint32_t teams = kI8Consumers / plan.per_row;
-    plan.share = 1;
-    for (uint32_t d = 2; d <= teams; ++d)
-        if (teams % d == 0 && d * kI8Rows * p.cols <= kI8StageCodes) plan.share = d;
-    plan.sets = teams / plan.share;
+    // Stages of 8 to 24 KB of codes: as many teams busy as can be, then the stage nearest to 16 KB. (With shares that divide the teams
+    // only, five teams over 1280 .. 1536 columns took stages of 5 KB: 21845 x 1536 16.3 us, 11.9 now, 15.0 with q8_i8_kernel.)
+    plan.share = teams, plan.sets = 1;  // narrow rows: no stage is large
+    uint32_t used = 0, off = 0;
+    for (uint32_t d = 1; d <= teams; ++d) {
+        const uint32_t codes = d * kI8Rows * p.cols, n = teams / d * d;
+        if (codes > kI8StageMax && d > 1) break;
+        const uint32_t o = codes < kI8StageBest ? kI8StageBest - codes : codes - kI8StageBest;
+        if (codes >= kI8StageMin && (n > used || (n == used && o < off))) plan.share = d, plan.sets = teams / d, used = n, off = o;
+    }
     plan.stage_bytes = plan.share * kI8Rows * (p.cols + 8 * gpr);  // a multiple of 16; at most 48 KB
     plan.stages = std::min<uint32_t>(kI8MaxStages, kI8Ring / plan.stage_bytes) / plan.sets * plan.sets;
     const uint32_t batches = (p.rows + kI8Rows - 1) / kI8Rows, blocks = std::min<uint32_t>(batches, (uint32_t)rt->sm_count);
@@ -476,10 +486,11 @@ Result gemv_q8(TesslRuntime *rt, const TesslBuf &packed, const TesslBuf &scales,
     const bool vec = group_size % 16 == 0 && cols % 16 == 0 && ((uintptr_t)packed.ptr & 15u) == 0 &&
                      ((uintptr_t)x.ptr & 15u) == 0 && cols > 0;
     if (vec) {
-        // The tables of every fourth row start at 16-byte boundaries if the buffers do. Below a megabyte of codes the start of the
-        // ring costs more than it gives: 512 x 1024 2.35 us without it, 2.55 with it; 513 x 4096 2.8 / 2.6.
+        // The tables of every fourth row start at 16-byte boundaries if the buffers do. For small calls the start of the ring costs more
+        // than it gives: 512 x 1024 2.35 us without it, 2.55 with it, 513 x 4096 2.8 / 2.6; 192 x 8192 3.0 / 3.4, 384 x 8192 4.0 / 3.7.
         const uint32_t warps = i8_warps_per_row(cols);
-        if (cols <= kI8MaxCols && weights >= (1u << 20) && (((uintptr_t)scales.ptr | (uintptr_t)zeros.ptr) & 15u) == 0)
+        const uint64_t least = cols <= 4096 ? 1u << 20 : 2u << 20;
+        if (cols <= kI8MaxCols && weights >= least && (((uintptr_t)scales.ptr | (uintptr_t)zeros.ptr) & 15u) == 0)
             return launch_i8_stream(rt, p);
         // Blocks of up to four warps have instantiations of their own: with a bound of 256 threads the compiler schedules the loop
         // differently, and 21 x 12288 took 4.4 us instead of 4.2.
