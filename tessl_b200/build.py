@@ -19,7 +19,7 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 LIB = HERE / "_lib" / "libtessl_b200.so"
 STEP_DRIVER = HERE / "_lib" / "tessl_step_driver"
-PY_CALL = HERE / "_lib" / "_tessl_call.so"
+PY_CALL = HERE / "_lib" / ("_tessl_call" + sysconfig.get_config_var("EXT_SUFFIX"))  # of this interpreter
 SOURCES = ["capi.cu", "nn_q4.cu", "nn_q8.cu", "q4_weight.cu", "prefill_gemm.cu", "peer_gather.cu", "qwen35_norm.cu", "mlx_q4_loader.cu"]
 
 
@@ -30,19 +30,31 @@ def nvcc_path() -> str:
     raise RuntimeError("nvcc not found (set NVCC or add it to PATH)")
 
 
+HEADER = HERE.parent / "include" / "tessl_b200.h"
+
+
+def _older(built, deps) -> bool:
+    return not all(b.exists() for b in built) or any(d.stat().st_mtime > min(b.stat().st_mtime for b in built) for d in deps)
+
+
 def is_stale() -> bool:
-    built = (LIB, STEP_DRIVER, PY_CALL)
-    if not all(b.exists() for b in built):
-        return True
-    t = min(b.stat().st_mtime for b in built)
-    deps = [d for pattern in ("*.cu", "*.cuh", "*.h", "*.cpp", "*.c") for d in CSRC.glob(pattern)]
-    deps.append(HERE.parent / "include" / "tessl_b200.h")
-    return any(d.stat().st_mtime > t for d in deps)
+    deps = [d for pattern in ("*.cu", "*.cuh", "*.h", "*.cpp") for d in CSRC.glob(pattern)]
+    return _older((LIB, STEP_DRIVER), deps + [HEADER])
 
 
 def build(force: bool = False, verbose_ptxas: bool = False) -> Path:
-    if not force and not is_stale():
-        return LIB
+    if force or is_stale():
+        build_library(verbose_ptxas)
+    if force or _older((PY_CALL,), (CSRC / "py_call.c", HEADER)):
+        try:
+            build_py_call()
+        except RuntimeError as e:  # no C compiler, or no headers of this interpreter
+            sys.stderr.write(f"tessl_b200: operator calls from Python will go through ctypes: {e}\n")
+    return LIB
+
+
+def build_library(verbose_ptxas: bool = False) -> None:
+    """The CUDA library and the step driver."""
     LIB.parent.mkdir(parents=True, exist_ok=True)
     host_cxx = "/usr/bin/g++" if Path("/usr/bin/g++").exists() else None
     cmd = [nvcc_path(), "-std=c++17", "-O3", "-lineinfo", "-gencode", "arch=compute_100a,code=sm_100a",
@@ -60,8 +72,6 @@ def build(force: bool = False, verbose_ptxas: bool = False) -> Path:
     if verbose_ptxas:
         sys.stderr.write(r.stderr)
     build_step_driver(host_cxx)
-    build_py_call()
-    return LIB
 
 
 def build_step_driver(host_cxx=None) -> Path:

@@ -10,7 +10,9 @@ from __future__ import annotations
 import ctypes as C
 import importlib.machinery
 import importlib.util
+import sysconfig
 import threading
+import warnings
 from pathlib import Path
 
 ABI_VERSION = 1
@@ -19,7 +21,7 @@ ROW_MAJOR, INTERLEAVED4, B200_STAGED = 0, 1, 2
 GEMM_Q4_MLX_MAX_M = 8
 
 LIB_PATH = Path(__file__).resolve().parent / "_lib" / "libtessl_b200.so"
-CALL_PATH = LIB_PATH.parent / "_tessl_call.so"
+CALL_PATH = LIB_PATH.parent / ("_tessl_call" + sysconfig.get_config_var("EXT_SUFFIX"))  # built for this interpreter
 
 
 class TesslError(RuntimeError):
@@ -164,6 +166,11 @@ def load() -> C.CDLL:
 ERR_LEN = 1024
 
 
+# What the native call module has (csrc/py_call.c).
+NATIVE_OPERATORS = ("gemv_q4_mlx_simd", "gemv_q4_mlx_gate_up_silu", "gemv_q4_mlx_kv", "gemv_q4_mlx_qkv", "swiglu", "gemm_q4_mlx",
+                    "gemm_q4_mlx_tensorops", "gemv_q8", "gemm_q8_mlx", "embed_lookup_q4_mlx", "qwen35_rms_norm",
+                    "qwen35_residual_add", "qwen35_add_rms_norm")
+
 _fn_cache: dict = {}
 _err_local = threading.local()
 
@@ -184,20 +191,21 @@ def call(name: str, *args) -> None:
         raise TesslError(st, err.value.decode("utf-8", "replace"))
 
 
-_native = None
-
-
 def native():
     """The operator calls without ctypes (csrc/py_call.c), for the library that `load` returns. Each returns True when it made
-    the call and False when it could not read an argument; a refusal is a TesslError."""
-    global _native
-    if _native is None:
-        load()
-        if not CALL_PATH.exists():
-            raise ImportError(f"{CALL_PATH} is missing: build it with `python -m tessl_b200.build`")
-        loader = importlib.machinery.ExtensionFileLoader("_tessl_call", str(CALL_PATH))
-        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_tessl_call", loader))
-        loader.exec_module(mod)
-        mod.set_error(TesslError)
-        _native = mod
-    return _native
+    the call and False when it could not read an argument; a refusal is a TesslError. None, with a warning, where the module was not
+    built for this interpreter and ABI: the callers' ctypes path serves every call."""
+    load()
+    if not CALL_PATH.exists():
+        warnings.warn(f"{CALL_PATH} is missing: operator calls go through ctypes, about 2 us more each "
+                      "(build it with `python -m tessl_b200.build`)", RuntimeWarning, stacklevel=2)
+        return None
+    loader = importlib.machinery.ExtensionFileLoader("_tessl_call", str(CALL_PATH))
+    mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_tessl_call", loader))
+    loader.exec_module(mod)
+    if mod.ABI_VERSION != ABI_VERSION:
+        warnings.warn(f"{CALL_PATH} has ABI {mod.ABI_VERSION}, this binding has {ABI_VERSION}: operator calls go through ctypes",
+                      RuntimeWarning, stacklevel=2)
+        return None
+    mod.set_error(TesslError)
+    return mod

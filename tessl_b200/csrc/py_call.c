@@ -299,5 +299,7 @@ PyMODINIT_FUNC PyInit__tessl_call(void)
     for (size_t i = 0; i < sizeof names / sizeof names[0]; ++i)
         if (!(*names[i].at = PyUnicode_InternFromString(names[i].name))) return NULL;
     error_class = Py_NewRef(PyExc_RuntimeError);
-    return PyModule_Create(&module);
+    PyObject *m = PyModule_Create(&module);
+    if (m && PyModule_AddIntConstant(m, "ABI_VERSION", TESSL_B200_ABI_VERSION) < 0) Py_CLEAR(m);
+    return m;
 }

@@ -221,12 +221,14 @@ def _opt(buf: Optional[GpuBuffer]):
 
 
 class _Native:
-    """The native calls, bound on first use: importing this module does not need the library."""
+    """The native calls, bound on first use: importing this module does not need the library. Where the native module is not there,
+    calls that say of every argument that they cannot read it."""
 
     def __getattr__(self, name):
-        fn = getattr(capi.native(), name)
-        setattr(self, name, fn)
-        return fn
+        mod = capi.native()
+        for op in capi.NATIVE_OPERATORS:
+            setattr(self, op, getattr(mod, op) if mod else lambda *args: False)
+        return getattr(self, name)
 
 
 _native = _Native()

@@ -74,3 +74,48 @@ def test_integers_wrap_as_ctypes_arguments_do():
     for n in (-1, 2**32, 2**40 + 3):
         with pytest.raises(nn.TesslError, match="null runtime handle"):
             nn.swiglu(NullRuntime(), B, B, B, n, False)
+
+
+def test_the_module_has_what_the_binding_calls():
+    native = capi.native()
+    assert native.ABI_VERSION == capi.ABI_VERSION
+    assert sorted(capi.NATIVE_OPERATORS) == sorted(CALLS) and all(callable(getattr(native, n)) for n in CALLS)
+
+
+@pytest.mark.parametrize("name", sorted(CALLS))
+def test_without_the_module_every_call_goes_through_ctypes(name, monkeypatch, tmp_path):
+    """A module that was not built, or only for another interpreter, whose file has another name."""
+    import shutil
+
+    shutil.copy(capi.CALL_PATH, tmp_path / "_tessl_call.cpython-27-elsewhere.so")
+    monkeypatch.setattr(capi, "CALL_PATH", tmp_path / capi.CALL_PATH.name)
+    monkeypatch.setattr(nn, "_native", nn._Native())
+    fn, args = CALLS[name]
+    with pytest.warns(RuntimeWarning, match="through ctypes"), pytest.raises(nn.TesslError, match="null runtime handle"):
+        fn(NullRuntime(), *args)
+    with pytest.raises(AttributeError):
+        fn(object(), *args)
+
+
+def test_a_module_of_another_abi_is_not_used(monkeypatch):
+    monkeypatch.setattr(capi, "ABI_VERSION", capi.ABI_VERSION + 1)
+    with pytest.warns(RuntimeWarning, match="has ABI"):
+        assert capi.native() is None
+
+
+def test_the_build_goes_on_without_the_module(monkeypatch, tmp_path, capsys):
+    from tessl_b200 import build
+
+    monkeypatch.setattr(build, "is_stale", lambda: False)
+    monkeypatch.setattr(build, "PY_CALL", tmp_path / "absent")
+    monkeypatch.setattr(build, "build_py_call", lambda: (_ for _ in ()).throw(RuntimeError("no C compiler found")))
+    assert build.build() == build.LIB
+    assert "ctypes: no C compiler found" in capsys.readouterr().err
+
+
+def test_another_interpreter_builds_its_own_module():
+    import sysconfig
+
+    from tessl_b200 import build
+
+    assert build.PY_CALL == capi.CALL_PATH and build.PY_CALL.name.endswith(sysconfig.get_config_var("EXT_SUFFIX"))
