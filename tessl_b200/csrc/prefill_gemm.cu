@@ -67,23 +67,29 @@ using nn::OUT_BF16;
 /// produces on the B side), then the per-group sums as (h1, h2, h3, h1) f16
 /// quadruples, then zero padding. a_aug is [M, K_aug] row-major.
 ///
-/// A thread holds its NC chunks of 8 elements in registers between the two passes, and the block is as wide as the row asks for:
-/// one round trip to memory and one barrier per row. (256 threads that read the row twice, in steps: 77 rows of 12288
-/// 4.4 us, of 1024 1.9 us.) NC = 0: rows too long for that, read twice.
-constexpr uint32_t kPrepMaxThreads = 768;
+/// A thread holds its NC chunks of 8 elements in registers between the two passes: one round trip to memory and one barrier per row.
+/// NC = 0: rows read twice.
+///
+/// Bound by latency up to some hundred rows, where a block is as wide as the row asks for, up to 768 threads. From there bound by memory
+/// (8192 rows of 14336: 3.4 TB/s in and out), and what it takes is rows in flight: blocks of 256 threads with up to eight chunks each, four
+/// on an SM, and past that rows read twice by eight blocks, out of L1 the second time: with the large carve-out of the others
+/// L1 would not hold them. Call of 64 weight rows, us, all rows read twice by 256 threads / all by wide blocks / here: 77 x 12288 48.4 / 46.7 /
+/// 46.7, 2048 x 6144 36.7 / 39.1 / 35.7, 2048 x 14336 80.6 / 92.4 / 80.4, 2048 x 17408 99 / 108 / 99, 8192 x 4096 48.0 / 49.0 / 45.0, 8192 x 14336
+/// 141 / 200 / 143.
+constexpr uint32_t kPrepMaxThreads = 768, kPrepManyThreads = 256, kPrepHeld = 8;
 
-template <int NC>
-__global__ void __launch_bounds__(kPrepMaxThreads) x_prepare_kernel(const uint16_t *x, __half *a_aug, float *row_scale, uint32_t K,
-                                                                    uint32_t K64, uint32_t K_aug, uint32_t gshift)
+template <int NC, int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == kPrepMaxThreads ? 2 : NC > 0 ? 4 : 8) x_prepare_kernel(const uint16_t *x, __half *a_aug, float *row_scale,
+                                                                                   uint32_t K, uint32_t K64, uint32_t K_aug, uint32_t gshift)
 {
     // Wait first, then let the GEMM start: its blocks set themselves up and stream weights while these rows are converted,
     // and everything in front of this kernel is complete when they do (2 - 4 us per call).
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const uint32_t m = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = blockDim.x;
+    const uint32_t m = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = NC > 0 ? blockDim.x : THREADS;
     const uint16_t *xrow = x + (size_t)m * K;
     __half *arow = a_aug + (size_t)m * K_aug;
-    __shared__ uint32_t red[kPrepMaxThreads / 32];
+    __shared__ uint32_t red[THREADS / 32];
 
     // largest magnitude (bf16 bit patterns order like integers); Inf/NaN disable the rescale
     constexpr int HELD = NC > 0 ? NC : 1;
@@ -633,12 +639,24 @@ Result prefill_launch(TesslRuntime *rt, const TesslQ4MlxBank &bank, const TesslB
     float *row_scale = reinterpret_cast<float *>(static_cast<char *>(scratch) + pl.a_bytes);
     SplitPlan sp;
     if (rt->prefill_force_split > 0) TESSL_TRY(split_plan(rt, m, pl, &sp));  // may refuse: before any launch
-    const uint32_t chunks = pl.k64 / 8, per = (chunks + kPrepMaxThreads - 1) / kPrepMaxThreads;  // chunks per thread
-    const auto prep = per == 1 ? x_prepare_kernel<1> : per == 2 ? x_prepare_kernel<2> : x_prepare_kernel<0>;
-    const uint32_t threads = per > 2 ? kPrepMaxThreads : ((chunks + per - 1) / per + 31) & ~31u;
+    const uint32_t chunks = pl.k64 / 8;
+    const bool many = m > 2 * (uint32_t)rt->sm_count;
+    // 8192 rows of 10240: held 107.5 us, read twice 102.7; 2048 of 12288 67.6 / 68.8
+    const bool twice = many && (pl.k > 16384 || (pl.k > 8192 && m >= 3072));
+    const uint32_t block = many ? kPrepManyThreads : kPrepMaxThreads;
+    const uint32_t per = (chunks + block - 1) / block;  // chunks per thread
+    const auto prep = twice      ? x_prepare_kernel<0, kPrepManyThreads>
+                      : per <= 1 ? x_prepare_kernel<1, kPrepMaxThreads>
+                      : per <= 2 ? x_prepare_kernel<2, kPrepMaxThreads>
+                      : !many    ? x_prepare_kernel<0, kPrepMaxThreads>
+                      : per <= 3 ? x_prepare_kernel<3, kPrepManyThreads>
+                      : per <= 4 ? x_prepare_kernel<4, kPrepManyThreads>
+                      : per <= 6 ? x_prepare_kernel<6, kPrepManyThreads>
+                                 : x_prepare_kernel<kPrepHeld, kPrepManyThreads>;
+    const uint32_t threads = twice || (!many && per > 2) ? block : ((chunks + per - 1) / per + 31) & ~31u;
     // The GEMM takes most of an SM's shared memory, and an SM changes its split of L1 and shared memory only when it is empty:
     // with the default split the GEMM's blocks could not start on the SMs that hold rows of the pre-pass.
-    TESSL_TRY(smem_opt_in(rt, reinterpret_cast<const void *>(prep), 0, "gemm_q4_mlx_tensorops: pre-pass", true));
+    if (!twice) TESSL_TRY(smem_opt_in(rt, reinterpret_cast<const void *>(prep), 0, "gemm_q4_mlx_tensorops: pre-pass", true));
     TESSL_TRY(launch_pdl(rt, "gemm_q4_mlx_tensorops pre-pass launch", prep, dim3(m), dim3(threads), 0,
                          static_cast<const uint16_t *>(x_bf16.ptr), a_aug, row_scale, pl.k, pl.k64, pl.k_aug, pl.gshift));
 

@@ -270,6 +270,36 @@ def test_dequant_groups_keep_their_stages_across_tiles(rt, tile, k, group):
         b.free()
 
 
+@pytest.mark.parametrize("k", [1024, 2112, 6144, 6208, 8192, 12288, 16384, 16448])
+@pytest.mark.parametrize("m", [297, 3072])
+def test_the_pre_pass_among_many_rows(rt, m, k):
+    """The forms that hold a row in one to eight pieces per thread or read it twice, which the pre-pass picks by the number of rows: the
+    bits of a call of a few rows, rows of all magnitudes, zeros and infinities included."""
+    n, group = 24, 64
+    packed, sb = synth.q4_bank(0x7E553800 + k, n, k, group)
+    bank = upload_bank(rt, packed.view(np.uint8).reshape(-1), sb.reshape(-1))
+    base = synth.bf16_bits_to_f32(synth.normal_bf16(0x7E553801 + k, 9 * k)).reshape(9, k)
+    base = base * np.float32(2.0) ** np.array([0, 40, -40, 15, -100, 0, 3, 0, 120], np.float32)[:, None]
+    base[5], base[7, k - 3] = 0.0, np.inf
+    x = synth.f32_to_bf16_bits(np.tile(base, (m // 9 + 1, 1))[:m].astype(np.float32).reshape(-1))
+    shape, y, y9 = nn.QuantShape(n, k, group), seeded_f32(rt, m * n), seeded_f32(rt, 27 * n)
+    xb = rt.buffer_from(x)
+    rt.set_prefill_tile(128, 1)
+    try:
+        nn.gemm_q4_mlx_tensorops(rt, bank, xb, y, shape, m)
+        nn.gemm_q4_mlx_tensorops(rt, bank, xb.view(0, 27 * k * 2), y9, shape, 27)
+    finally:
+        rt.set_prefill_tile(0, -1)
+    got, few = y.read(np.uint32, m * n).reshape(m, n), y9.read(np.uint32, 27 * n).reshape(27, n)
+    assert np.array_equal(got, np.tile(few[:9], (m // 9 + 1, 1))[:m]) and np.array_equal(few[9:18], few[:9])
+    rows = [0, 1, 2, 3, 4, 6]
+    xs = np.ascontiguousarray(x.reshape(m, k)[rows]).reshape(-1)
+    want = api.q4_dense_gemm(packed.view(np.uint8).reshape(-1), sb.reshape(-1), xs, len(rows), n, k, group)
+    scale = np.float32(2.0) ** np.array([0, 40, -40, 15, -100, 3], np.float32)[:, None]
+    assert_north_star(few[rows].view(np.float32) / scale, want / scale, f"{m} rows of {k}")
+    assert not few[5].any() and not np.isfinite(few[7].view(np.float32)).any()
+
+
 def test_rows_of_any_magnitude_survive_the_f16_operands(rt):
     """The per-row power-of-two rescale: rows scaled by 2^-40 .. 2^+60 give the
     correspondingly scaled outputs, a zero row gives zeros."""
