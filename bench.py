@@ -15,7 +15,7 @@ weight bytes of the step / device time) with everything resident in HBM;
 `e2e` is the same measured by a compiled C++ host over the C ABI
 (tessl_b200/csrc/host_step_driver.cpp) with the activations copied from pinned
 host memory and the result read back every step (encode-only mode; the
-every-call-synchronous figure and the Python-ctypes figures beside it);
+every-call-synchronous figure and the figures from Python beside it);
 `roofline` describes the dominant kernel, `roofline_prefill` the prefill GEMM;
 `cpu_baseline` times the CPU oracle on the same workload; `parity` is the GPU
 step's result against the CPU arm's on the same banks (layer 0 of the GPU arm
@@ -708,7 +708,7 @@ def measure_sharded_lm_head(ctx, args, world, rank):
 
 
 def measure_e2e_python(ctx, args):
-    """The step through the C ABI from Python (ctypes): activations copied from pinned host memory each
+    """The step through the C ABI from Python (tessl_b200.nn): activations copied from pinned host memory each
     step, the down projection's output read back each step. Timed in encode-only mode and with every
     call synchronous. What an interpreter adds to the compiled host's figure."""
     torch, nn, rt = ctx["torch"], ctx["nn"], ctx["rt"]
@@ -793,7 +793,7 @@ def measure_e2e(ctx, args, device: int):
             "value_every_call_synchronous": d["value_every_call_synchronous"],
             "ms_per_step_synchronous": d["ms_per_step_synchronous"],
             "first_result_vs_this_process": "bit-exact" if same else f"max |diff| {diff:.3g}",
-            "python_ctypes": {k: py[k] for k in ("value", "ms_per_step", "value_every_call_synchronous",
+            "python_binding": {k: py[k] for k in ("value", "ms_per_step", "value_every_call_synchronous",
                                                  "ms_per_step_synchronous", "steps")}}
 
 

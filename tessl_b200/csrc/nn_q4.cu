@@ -1106,10 +1106,11 @@ Result swiglu(TesslRuntime *rt, const TesslBuf &gate, const TesslBuf &up, const 
                          out_as_bf16 ? 1 : 0, 0);
 }
 
-/// A validated prefill call with few rows, run as batches of up to 8 rows on the tensor-core GEMV kernel:
-/// up to 24 rows that is faster than the prefill GEMM, whose 256-row tile would be mostly padding (24 rows as three
-/// batches against 25 through the GEMM: 12288 x 4096 23.8 / 33.2 us, 4096 x 4096 13.9 / 22.0, 2048 x 2048 8.1 / 13.3, 1024 x
-/// 1024 6.7 / 9.7). At the widths where a single row has the tensor-core kernel; `*handled` is false at the others.
+/// A validated prefill call with few rows, run as batches of up to 8 rows on the tensor-core GEMV kernel, at the widths where a
+/// single row has the tensor-core kernel; `*handled` is false at the others. One or two batches are faster than the prefill GEMM's
+/// 25 rows everywhere (16 rows / 25 rows, us: 12288 x 4096 15.9 / 18.9, 4096 x 4096 9.1 / 11.4, 2048 x 2048 5.2 / 8.2, 1024 x 1024 4.2 /
+/// 8.1). Three batches were, too, against the GEMM of 256-row tiles that the line at 24 was drawn for; against the split
+/// kernel they lose at the wide calls (24 rows: 23.3, 13.3, 7.7, 6.2 us).
 Result prefill_as_small_batches(TesslRuntime *rt, const TesslQ4MlxBank &bank, const TesslBuf &x_bf16, const TesslBuf &y,
                                 const TesslQuantShape &shape, uint32_t m, OutKind out, bool *handled)
 {

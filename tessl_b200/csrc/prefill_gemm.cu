@@ -79,8 +79,8 @@ using nn::OUT_BF16;
 constexpr uint32_t kPrepMaxThreads = 768, kPrepManyThreads = 256, kPrepHeld = 8;
 
 template <int NC, int THREADS>
-__global__ void __launch_bounds__(THREADS, THREADS == kPrepMaxThreads ? 2 : NC > 0 ? 4 : 8) x_prepare_kernel(const uint16_t *x, __half *a_aug, float *row_scale,
-                                                                                   uint32_t K, uint32_t K64, uint32_t K_aug, uint32_t gshift)
+__global__ void __launch_bounds__(THREADS, THREADS == kPrepMaxThreads ? 2 : NC > 0 ? 4 : 8)
+    x_prepare_kernel(const uint16_t *x, __half *a_aug, float *row_scale, uint32_t K, uint32_t K64, uint32_t K_aug, uint32_t gshift)
 {
     // Wait first, then let the GEMM start: its blocks set themselves up and stream weights while these rows are converted,
     // and everything in front of this kernel is complete when they do (2 - 4 us per call).
@@ -489,14 +489,15 @@ Result prefill_validate(const TesslQ4MlxBank &bank, const TesslBuf &x_bf16, cons
     return ok();
 }
 
-/// The pair kernel's 256-row tile is half padding for m <= 128, but each CTA still expands only half of
-/// the weight rows and it has the better pipeline: measured 34.6 us against the single-CTA kernel's 48.9 us
-/// at m = 16 .. 64, N = 12288, K = 4096. So the pair kernel runs for every m; the single-CTA kernel is
-/// what a GPU with one SM, or `tessl_runtime_set_prefill_tile(rt, bn, 0)`, selects.
+/// Few rows of X are the split kernel's (prefill_launch), all others the pair kernel's. Its 256-row tile is half padding for m <= 128, but
+/// each CTA expands only half of the weight rows and it has the better pipeline than the single-CTA kernel: 28.0 against 43.2 us at 16 x
+/// 12288 x 4096 (split kernel 19.2). The single-CTA kernel is what a GPU with one SM, or
+/// `tessl_runtime_set_prefill_tile(rt, bn, 0)`, selects.
 
 /// Tile width with the least estimated time: waves of tiles x the cost of one tile's K block. The 64-wide tile (pair kernel
-/// only) is for calls whose wider tiles leave clusters idle: 77 x 4096 x 12288 is 32 tiles of 128 on 74 clusters, 62.3 us,
-/// and 64 of 64, 52.7 us; 509 x 2048 x 6144 35.7 / 30.2 us, 257 x 1024 x 1024 10.3 / 9.1. What is left there is the chain of K blocks, 0.26 us each.
+/// only) is for calls whose wider tiles leave clusters idle: 509 x 2048 x 2048 is 32 tiles of 128 on 74 clusters, 15.1 us, and 64 of 64,
+/// 13.0 us; 257 x 1024 x 1024 9.8 / 8.6, 257 x 1999 x 1088 20.4 / 15.0; and the other way, 420 x 3072 x 1024 10.2 / 13.1. What is left there is
+/// the chain of K blocks, 0.26 us each.
 int pick_tile_width(uint64_t tiles_m, uint32_t n, uint32_t slots, bool pair)
 {
     int best_bn = 256;
@@ -518,10 +519,12 @@ struct SplitPlan {
     uint64_t cost = ~0ull;
 };
 
-/// At least this much shared memory keeps a second CTA off the SM. Each CTA holds all of its SM's TMEM: CTAs of two clusters
-/// that shared SMs crosswise would wait for each other's TMEM and never get it.
-constexpr uint32_t kSplitMinSmem = 120 * 1024;
-constexpr uint32_t kSplitMaxUsed = 6;  // 16 x 2048 rows in 6 / 8: clusters of 8 find room for 16 at most, two rounds from there
+/// At least this much shared memory keeps a second CTA of a kernel that uses TMEM off the SM. Each CTA holds all of its SM's TMEM: CTAs
+/// of two clusters that shared SMs crosswise would wait for each other's TMEM and never get it.
+constexpr uint32_t kSplitMinSmem = 120 * 1024, kSmemPerSm = 228 * 1024;
+constexpr uint32_t kLeastTmemSmem = std::min({kSplitMinSmem, PairCfg<64>::SMEM, PairCfg<128>::SMEM, PairCfg<192>::SMEM, PairCfg<256>::SMEM,
+                                              Cfg<128>::SMEM, Cfg<192>::SMEM, Cfg<256>::SMEM});
+static_assert(2 * kLeastTmemSmem > kSmemPerSm, "two CTAs on one SM would both want its TMEM");
 
 /// Clusters of `split` CTAs of the split kernel that the device holds at once (a cluster lies in one GPC: 45 of three, 33 of
 /// four, 26 of five, 22 of six). The kernel's shared memory has been opted in.
@@ -564,7 +567,7 @@ Result split_plan(TesslRuntime *rt, uint32_t m, const PrefillPlan &pl, SplitPlan
         best = SplitPlan{tiles_m, x_rows, s, 0};
         return ok();
     }
-    for (uint32_t s = 1; s <= kSplitMaxUsed && blocks >= 4 * s; ++s) {
+    for (uint32_t s = 1; s <= SplitCfg::MAX_SPLIT && blocks >= 4 * s; ++s) {
         const uint64_t room = (uint64_t)split_clusters(rt, s), waves = (tiles + room - 1) / room;
         const uint64_t part = (blocks + s - 1) / s;
         const uint64_t cost = waves * ((s > 1 ? 4500 : 5200) + 8 * x_rows + part * (2000 + 3 * x_rows) / 10) +

@@ -14,9 +14,9 @@
 //   * a lane holds one weight row of D, so 32 lanes store 32 neighbours of a row of y: whole lines without a transposition,
 //     for any N.
 //
-// What bounds it: per K block and SM 0.2 us, most of it the dequant warps' instructions (77 x 4096 x 12288 on 32 SMs: issue
-// slots 56 % busy, FMA and ALU pipes 39 % each, tensor pipe 39 %), then ~4 us around them (pre-pass, start, first copies,
-// last stores) and 2 - 3 us for the exchange of a cluster. On the way: one wait and one commit per unit instead of two rings
+// What bounds it: per K block and SM 0.2 us, most of it the dequant warps' instructions (77 x 4096 x 12288 in clusters of four, over
+// the whole launch: issue slots 41 % busy, ALU pipe 27 %, f16 FMA 19 %, tensor pipe 24 %), then ~4 us around them (pre-pass, start,
+// first copies, last stores) and 2 - 3 us for the exchange of a cluster. On the way: one wait and one commit per unit instead of two rings
 // and a commit per K block 0.25 -> 0.19 us per K block; row scales read once per CTA instead of by every epilogue warp from the
 // same lines of L2 9 -> 2 us per tile; scale words in the dequant threads' registers instead of copied by one warp 22.5 ->
 // 15.9 us at 100 x 1000 x 2080. Tried: two CTAs per SM with half the TMEM each (the scheduler packs them on half of the SMs:
@@ -44,7 +44,7 @@ struct SplitCfg {
     static constexpr int NG = 4;           // dequant groups of four warps; group g expands units g, g + NG, ...
     static constexpr int SQ = 8;           // packed stages, a unit (two K blocks) each
     static constexpr int MAX_SU = 6;       // stages of (X tiles, expanded weights), a unit each
-    static constexpr int MAX_SPLIT = 8;
+    static constexpr uint32_t MAX_SPLIT = 6;  // CTAs per tile: clusters of eight find room for 16 at most
     static constexpr int FIRST_DW = 4;     // first dequant warp
     static constexpr int THREADS = (FIRST_DW + NG * 4) * 32;
     static constexpr uint32_t UNIT_COLS = 64;           // TMEM columns of an expanded unit
